@@ -30,6 +30,29 @@ class AuxSide(ctypes.Structure):
     _fields_ = [(n, ctypes.c_void_p) for n in ("cxyz", "pstart", "nprim", "pexp", "pcoef", "rexp", "aostart", "atom")]
 
 
+class Bra(ctypes.Structure):
+    _fields_ = [(n, ctypes.c_void_p) for n in (
+        "shA", "shB", "pstart", "npair", "rec", "cxyz", "aostart", "atom")] + [("b_dummy", ctypes.c_int)]
+
+
+class Groups(ctypes.Structure):
+    _fields_ = [(n, ctypes.c_void_p) for n in ("info", "coef", "shells", "pexp", "rexp", "cxyz", "aostart", "atom")]
+
+
+class GradClass(ctypes.Structure):
+    _fields_ = [("la", ctypes.c_int), ("lb", ctypes.c_int), ("lc", ctypes.c_int), ("npair", ctypes.c_int),
+                ("pairs", ctypes.c_void_p), ("chunks", ctypes.c_void_p), ("nchunk", ctypes.c_int),
+                ("nq", ctypes.c_int)]
+
+
+class PrimClass(ctypes.Structure):
+    _fields_ = [("la", ctypes.c_int), ("lb", ctypes.c_int), ("lc", ctypes.c_int), ("npair", ctypes.c_int),
+                ("pairs", ctypes.c_void_p), ("chunks", ctypes.c_void_p), ("groups", ctypes.c_void_p),
+                ("rows", ctypes.c_void_p), ("first_chunk", ctypes.c_void_p), ("ngroup", ctypes.c_int),
+                ("max_shells", ctypes.c_int), ("bra_groups", ctypes.c_void_p), ("nbra_groups", ctypes.c_int), ("bra_prim0", ctypes.c_int),
+                ("f32", ctypes.c_int)]
+
+
 _SIGS = {
     "dfb_version": (ctypes.c_int, []),
     "dfb_last_error": (ctypes.c_char_p, []),
@@ -61,6 +84,19 @@ _SIGS = {
     "dfb_gamma_sym": (ctypes.c_int, [ctypes.c_long, ctypes.c_int, ctypes.c_int, _d, ctypes.c_long, ctypes.c_long,
                                      _d, _d, _d]),
     "dfb_fp32_fma_probe": (ctypes.c_int, [_d, ctypes.c_int, ctypes.c_int, ctypes.c_int, _d]),
+    "dfb_pair_ext": (ctypes.c_int, [_d] * 7 + [ctypes.c_long, _d, _d]),
+    "dfb_fork": (ctypes.c_int, [_d, ctypes.POINTER(ctypes.c_void_p), ctypes.c_int]),
+    "dfb_join": (ctypes.c_int, [_d, ctypes.POINTER(ctypes.c_void_p), ctypes.c_int]),
+    "dfb_grad_supported": (ctypes.c_int, [ctypes.c_int] * 4),
+    "dfb_grad_contract": (ctypes.c_int, [ctypes.POINTER(Bra), ctypes.POINTER(Groups), ctypes.POINTER(GradClass),
+                                         ctypes.c_int, _d, ctypes.c_long, ctypes.c_long, ctypes.c_long, _d,
+                                         ctypes.c_int, ctypes.POINTER(ctypes.c_void_p), ctypes.c_int]),
+    "dfb_prim_scratch": (ctypes.c_long, [ctypes.POINTER(PrimClass), ctypes.c_int, ctypes.c_long]),
+    "dfb_prim_integrals": (ctypes.c_int, [ctypes.POINTER(Bra), ctypes.POINTER(Groups), ctypes.POINTER(PrimClass),
+                                          ctypes.c_int, _d, ctypes.c_long, ctypes.c_long, ctypes.c_long, _d,
+                                          ctypes.c_long, ctypes.POINTER(ctypes.c_void_p), ctypes.c_int]),
+    "dfb_zero_pairs": (ctypes.c_int, [ctypes.POINTER(Bra), _d, ctypes.c_int, _d, ctypes.c_long, _d, ctypes.c_long,
+                                      ctypes.c_long, ctypes.c_long, _d]),
     "dfb_launch_count": (ctypes.c_long, []),
     "dfb_rys_scratch_doubles": (ctypes.c_long, [ctypes.c_int] * 3 + [ctypes.c_long, ctypes.c_int]),
     "dfb_fp64_fma_probe": (ctypes.c_int, [_d, ctypes.c_int, ctypes.c_int, ctypes.c_int, _d]),

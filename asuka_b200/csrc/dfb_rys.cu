@@ -577,6 +577,11 @@ static int current_device() {
     return dev;
 }
 
+const RysTable* rys_table_of_current_device() {
+    const int dev = current_device();
+    return dev >= 0 && dev < 64 && g_tables[dev].ready ? &g_tables[dev].tab : nullptr;
+}
+
 // Scratch policy of the generic path: one slot (nef or 3 nef doubles) per task
 // of a batch; batches of up to DFB_SCRATCH_TASKS tasks, or fewer when the
 // caller's scratch is smaller (the fixed scratch of dfb_rys_int_noalloc).

@@ -32,12 +32,16 @@ import torch
 
 from . import _lib
 from . import linalg as _la
+from .auxgroups import AuxGroups, DevicePool
 from .basis import BasisCartSoA, build_shell_pairs_l_order, from_reference_like, ncart
 
 _DATA = os.path.join(os.path.dirname(os.path.abspath(__file__)), "data")
 _TABLE_READY: set[int] = set()
 PRIM_SCREEN = 1e-20  # primitive-pair magnitude bound below which a pair is skipped (0 = evaluate all)
 NSTREAMS = int(os.environ.get("DFB_STREAMS", "8"))  # side streams for per-class launches (2/4/6/8 measured: 8 fastest)
+PRIM_WAVE = 1 << 23  # doubles of primitive integrals per stream and wave of a class (64 MB)
+GRAD_THREADS = 1 << 19  # lanes of one derivative class below which its tasks are single primitives
+SEG_PRIMS = 4  # primitive pairs of a derivative task: contracted pairs are cut, so that no task outlasts the rest
 NROOTS_SLOTS = 11  # DFB_NROOTS_MAX + 1
 _SIDE_STREAMS: dict[int, list] = {}
 
@@ -109,10 +113,11 @@ def _prec_code(precision: str) -> int:
 
 @functools.lru_cache(maxsize=1)
 def mixed_class_table() -> dict:
-    """Angular classes whose FP32-component kernels the mixed mode uses, per kind ('int3c',
-    'deriv3c', 'deriv2c'), as sets of (la, lb, lc).  Written by ``asuka_b200.tune_precision``
-    from the measured first-order energy and gradient errors of every class (FP32 against FP64
-    kernels); classes not listed run in FP64 in mixed mode too."""
+    """Angular classes whose FP32-component kernels the mixed mode uses, per kind, as sets of
+    (la, lb, lc).  Written by ``asuka_b200.tune_precision`` from the measured first-order energy and
+    gradient errors of every class (FP32 against FP64 kernels); classes not listed run in FP64 in
+    mixed mode too.  The mixed mode reads 'int3c': its derivative contractions run on the FP64 group
+    kernels, which are faster than the FP32 shell kernels ('deriv3c' and 'deriv2c' were measured for those)."""
     p = os.path.join(_DATA, "class_precision.json")
     if not os.path.exists(p):
         return {}
@@ -164,61 +169,66 @@ class DFEngine:
         if ao.lmax > 8 or aux.lmax > 8:
             raise NotImplementedError("shells with l > 8 are not supported")
         dev = self.device
-        i32 = self._i32
-        f64 = self._f64
 
-        # ---- AO side: basis arrays and l-ordered shell pairs
+        # ---- AO side (basis arrays, l-ordered shell pairs) and aux side, one upload per type
         self.sp = build_shell_pairs_l_order(ao)
-        self.ao_cxyz = f64(ao.shell_cxyz)
-        self.ao_pstart = i32(ao.shell_prim_start)
-        self.ao_nprim = i32(ao.shell_nprim)
-        self.ao_exp = f64(ao.prim_exp)
-        self.ao_coef = f64(ao.prim_coef)
-        self.ao_aostart = i32(ao.shell_ao_start)
-        self.ao_atom = i32(ao.shell_atom)
-        self.sp_A = i32(self.sp.sp_A)
-        self.sp_B = i32(self.sp.sp_B)
-
-        # ---- aux side: basis arrays and (P, dummy) self-pair tables for the metric
-        self.ax_cxyz = f64(aux.shell_cxyz)
-        self.ax_pstart = i32(aux.shell_prim_start)
-        self.ax_nprim = i32(aux.shell_nprim)
-        self.ax_exp = f64(aux.prim_exp)
-        self.ax_coef = f64(aux.prim_coef)
-        self.ax_rexp = f64(1.0 / np.asarray(aux.prim_exp, dtype=np.float64))
-        self.ax_aostart = i32(aux.shell_ao_start)
-        self.ax_atom = i32(aux.shell_atom)
-        self.ax_self = i32(np.arange(aux.nshell, dtype=np.int32))
-        self.ax_pp_sp = i32(np.repeat(np.arange(aux.nshell, dtype=np.int32), aux.shell_nprim))
+        ints, dbls = DevicePool(np.int32), DevicePool(np.float64)
+        aux_l = aux.shell_l
+        ilist = [ao.shell_prim_start, ao.shell_nprim, ao.shell_ao_start, ao.shell_atom, self.sp.sp_A, self.sp.sp_B,
+                 aux.shell_prim_start, aux.shell_nprim, aux.shell_ao_start, aux.shell_atom, np.arange(aux.nshell),
+                 np.repeat(np.arange(aux.nshell), aux.shell_nprim)]
+        by_l = {}
+        for l in np.unique(aux_l):
+            idx = np.nonzero(aux_l == l)[0]
+            by_l[int(l)] = ints.add(idx[np.argsort(-aux.shell_nprim[idx], kind="stable")])
+        ih = [ints.add(a) for a in ilist]
+        dh = [dbls.add(a) for a in (ao.shell_cxyz, ao.prim_exp, ao.prim_coef, aux.shell_cxyz, aux.prim_exp, aux.prim_coef,
+                                    1.0 / np.asarray(aux.prim_exp, dtype=np.float64))]
+        di, dd = ints.upload(dev), dbls.upload(dev)
+        (self.ao_pstart, self.ao_nprim, self.ao_aostart, self.ao_atom, self.sp_A, self.sp_B, self.ax_pstart,
+         self.ax_nprim, self.ax_aostart, self.ax_atom, self.ax_self, self.ax_pp_sp) = (di(h) for h in ih)
+        (self.ao_cxyz, self.ao_exp, self.ao_coef, self.ax_cxyz, self.ax_exp, self.ax_coef,
+         self.ax_rexp) = (dd(h) for h in dh)
+        self.aux_by_l = {l: di(h) for l, h in by_l.items()}
+        # (P, dummy) self-pair tables of the shell-by-shell metric kernels
         self.axpt = torch.empty((7, max(int(aux.shell_nprim.sum()), 1)), dtype=torch.float64, device=dev)
         self.ps_aux = _lib.PairSide(
             *[_lib.ptr(t) for t in (self.ax_self, self.ax_self, self.ax_pstart, self.ax_nprim, *self.axpt,
                                     self.ax_cxyz, self.ax_aostart, self.ax_atom)], 1)
         self.axs = _lib.AuxSide(*[_lib.ptr(t) for t in (self.ax_cxyz, self.ax_pstart, self.ax_nprim, self.ax_exp,
                                                         self.ax_coef, self.ax_rexp, self.ax_aostart, self.ax_atom)])
-        aux_l = aux.shell_l
-        self.aux_by_l = {}
-        for l in np.unique(aux_l):
-            idx = np.nonzero(aux_l == l)[0]
-            idx = idx[np.argsort(-aux.shell_nprim[idx], kind="stable")]
-            self.aux_by_l[int(l)] = i32(idx)
-        # metric classes: unordered aux pairs oriented l(P) >= l(Q)
-        self.classes2c = []
-        nsh = aux.nshell
-        Pi, Qi = np.tril_indices(nsh)
-        lp, lq = aux_l[Pi], aux_l[Qi]
-        swap = lp < lq
-        P = np.where(swap, Qi, Pi)
-        Q = np.where(swap, Pi, Qi)
-        lP, lQ = aux_l[P], aux_l[Q]
-        for a in np.unique(lP):
-            for c in np.unique(lQ):
-                sel = np.nonzero((lP == a) & (lQ == c))[0]
-                if sel.size:
-                    self.classes2c.append((int(a), int(c), i32(P[sel]), i32(Q[sel])))
+        self._classes2c = None
+        self._epoch = 0
+        self.groups = AuxGroups(aux, np.arange(aux.nshell), dev, self.ax_cxyz, self.ax_aostart, self.ax_atom)
         self._scratch = scratch if scratch is not None else ScratchHolder()
         self._build_ao_pairs(ao.shell_cxyz)
         self._build_pair_tables()
+
+    # ------------------------------------------------------------ class lists
+    @property
+    def classes3c(self):
+        """(la, lb, lc, AO pair list, aux shell list) per angular class; assigning a list drops the launch plans."""
+        return self._classes3c
+
+    @classes3c.setter
+    def classes3c(self, classes) -> None:
+        self._classes3c = classes
+        self._epoch += 1
+
+    @property
+    def classes2c(self):
+        """Metric classes of the shell-by-shell kernels: (lP, lQ, P list, Q list) over the unordered aux shell
+        pairs oriented l(P) >= l(Q); built when first asked for."""
+        if self._classes2c is None:
+            aux_l = self.aux.shell_l
+            Pi, Qi = np.tril_indices(self.aux.nshell)
+            swap = aux_l[Pi] < aux_l[Qi]
+            P, Q = np.where(swap, Qi, Pi), np.where(swap, Pi, Qi)
+            lP, lQ = aux_l[P], aux_l[Q]
+            self._classes2c = [(int(a), int(c), self._i32(P[sel]), self._i32(Q[sel]))
+                               for a in np.unique(lP) for c in np.unique(lQ)
+                               if (sel := np.nonzero((lP == a) & (lQ == c))[0]).size]
+        return self._classes2c
 
     # ------------------------------------------------------------ class launches over streams
     def _streams(self):
@@ -229,23 +239,21 @@ class DFEngine:
             _SIDE_STREAMS[idx] = [torch.cuda.Stream(device=self.device) for _ in range(NSTREAMS)]
         return _SIDE_STREAMS[idx]
 
-    def _fanout(self, launches):
-        """Run launch(stream_ptr) callables round-robin over side streams, ordered after and
-        before the current stream."""
+    def _fork(self):
+        """(main stream, side streams, ctypes array of their handles), the side streams ordered after the
+        current stream."""
         main = torch.cuda.current_stream(self.device)
-        side = self._streams() if NSTREAMS > 1 else [main]
-        if NSTREAMS > 1:
-            start = torch.cuda.Event()
-            start.record(main)
-            for st in side:
-                st.wait_event(start)
-        for i, fn in enumerate(launches):
-            fn(int(side[i % len(side)].cuda_stream))
-        if NSTREAMS > 1:
-            for st in side:
-                ev = torch.cuda.Event()
-                ev.record(st)
-                main.wait_event(ev)
+        if NSTREAMS <= 1:
+            return main, [main], (ctypes.c_void_p * 1)(int(main.cuda_stream))
+        side = self._streams()
+        arr = (ctypes.c_void_p * len(side))(*[int(st.cuda_stream) for st in side])
+        _lib.check(_lib.lib().dfb_fork(int(main.cuda_stream), arr, len(side)), "dfb_fork")
+        return main, side, arr
+
+    def _join(self, fork) -> None:
+        main, side, arr = fork
+        if side[0] is not main:
+            _lib.check(_lib.lib().dfb_join(int(main.cuda_stream), arr, len(side)), "dfb_join")
 
     @property
     def _i32(self):
@@ -286,34 +294,55 @@ class DFEngine:
         cnt = np.bincount(kept_owner, minlength=sp.nsp).astype(np.int32)
         start = np.zeros(sp.nsp, dtype=np.int64)
         np.cumsum(cnt[:-1], out=start[1:])
-        i32 = self._i32
-        self.sp_pstart = i32(start)
-        self.sp_npair = i32(cnt)
-        self.pp_sp = i32(kept_owner)
-        self.pp_local = i32(loc[keep])
-        self.n_prim_pairs = int(keep.sum())
-        self.n_prim_pairs_total = int(owner.size)
-        self.pt = torch.empty((7, max(self.n_prim_pairs, 1)), dtype=torch.float64, device=self.device)
-        self.ps_ao = _lib.PairSide(
-            *[_lib.ptr(t) for t in (self.sp_A, self.sp_B, self.sp_pstart, self.sp_npair, *self.pt, self.ao_cxyz,
-                                    self.ao_aostart, self.ao_atom)], 0)
         la = ao.shell_l[sp.sp_A]
         lb = ao.shell_l[sp.sp_B]
         live = cnt > 0
-        # dropped shell pairs write nothing: outputs are zero-filled first when any exist
-        self.n_dropped_pairs = int((~live).sum())
-        self.classes3c = []  # (la, lb, lc, pairs tensor, aux tensor)
+        pool = DevicePool(np.int32)
+        hs = [pool.add(a) for a in (start, cnt, kept_owner, loc[keep])]
+        ph = {}
         for a in np.unique(la):
             for b in np.unique(lb):
                 sel = np.nonzero((la == a) & (lb == b) & live)[0]
-                if sel.size == 0:
-                    continue
-                # pairs by decreasing primitive-pair count: with the aux-major task
-                # grid a warp walks pairs of similar cost against one aux shell
-                sel = sel[np.argsort(-cnt[sel], kind="stable")]
-                pairs = i32(sel)
-                for c, auxs in self.aux_by_l.items():
-                    self.classes3c.append((int(a), int(b), int(c), pairs, auxs))
+                if sel.size:
+                    # pairs by decreasing primitive-pair count: with the aux-major task
+                    # grid a warp walks pairs of similar cost against one aux shell.  Equal
+                    # counts by (A, B): neighbouring pairs then read and write neighbouring
+                    # columns of one 3c row
+                    sel = sel[np.lexsort((sp.sp_B[sel], sp.sp_A[sel], -cnt[sel]))]
+                    ph[int(a), int(b)] = pool.add(sel)
+        # derivative bra entries: segments of at most SEG_PRIMS primitive pairs (their contributions add)
+        nseg = -(-cnt.astype(np.int64) // SEG_PRIMS)
+        seg_pair = np.repeat(np.arange(sp.nsp), nseg)
+        k = np.arange(seg_pair.size) - np.repeat(np.cumsum(nseg) - nseg, nseg)
+        seg_n = np.minimum(SEG_PRIMS, cnt[seg_pair] - SEG_PRIMS * k)
+        gs = [pool.add(a) for a in (sp.sp_A[seg_pair], sp.sp_B[seg_pair], start[seg_pair] + SEG_PRIMS * k, seg_n)]
+        gh = {}
+        for (a, b) in ph:
+            sel = np.nonzero((la[seg_pair] == a) & (lb[seg_pair] == b))[0]
+            gh[a, b] = pool.add(sel[np.lexsort((k[sel], sp.sp_B[seg_pair[sel]], sp.sp_A[seg_pair[sel]], -seg_n[sel]))])
+        hz, hn = pool.add(np.nonzero(~live)[0]), pool.add((ao.shell_l + 1) * (ao.shell_l + 2) // 2)
+        size = (ao.shell_l.astype(np.int64) + 1) * (ao.shell_l + 2) // 2
+        dropped = float((size[sp.sp_A] * size[sp.sp_B])[~live].sum()) * 2.0 / max(ao.nao, 1) ** 2
+        di = pool.upload(self.device)
+        self.sp_pstart, self.sp_npair, self.pp_sp, self.pp_local = (di(h) for h in hs)
+        self._dropped = (di(hz), di(hn), dropped)  # pairs without primitives, shell sizes, their share of a 3c row
+        self._segs = tuple(di(h) for h in gs)
+        self._seg_lists = {key: di(h) for key, h in gh.items()}
+        self.n_prim_pairs = int(keep.sum())
+        self.n_prim_pairs_total = int(owner.size)
+        self.pt = torch.empty((7, max(self.n_prim_pairs, 1)), dtype=torch.float64, device=self.device)
+        self.prec = torch.empty((max(self.n_prim_pairs, 1), 8), dtype=torch.float64, device=self.device)
+        p = _lib.ptr
+        rest = (p(self.prec), p(self.ao_cxyz), p(self.ao_aostart), p(self.ao_atom), 0)
+        self.bra_ao = _lib.Bra(p(self.sp_A), p(self.sp_B), p(self.sp_pstart), p(self.sp_npair), *rest)
+        self.bra_seg = _lib.Bra(*[p(t) for t in self._segs], *rest)
+        self.ps_ao = _lib.PairSide(
+            *[_lib.ptr(t) for t in (self.sp_A, self.sp_B, self.sp_pstart, self.sp_npair, *self.pt, self.ao_cxyz,
+                                    self.ao_aostart, self.ao_atom)], 0)
+        # dropped shell pairs write nothing: outputs are zero-filled first when any exist
+        self.n_dropped_pairs = int((~live).sum())
+        self.classes3c = [(a, b, c, pairs, auxs) for (a, b), pairs in ((k, di(h)) for k, h in ph.items())
+                          for c, auxs in self.aux_by_l.items()]  # (la, lb, lc, pairs tensor, aux tensor)
         self._aux_blocks_n = None
 
     # ------------------------------------------------------------ helpers
@@ -325,6 +354,8 @@ class DFEngine:
                                p(self.sp_A), p(self.sp_B), p(self.sp_pstart), p(self.pp_sp), p(self.pp_local), npp, 0,
                                *[p(r) for r in self.pt], _stream())
         _lib.check(rc, "dfb_pair_tables(ao)")
+        eta, px, py, pz, ck, ea, eb = (p(r) for r in self.pt)
+        _lib.check(L.dfb_pair_ext(eta, px, py, pz, ck, ea, eb, npp, p(self.prec), _stream()), "dfb_pair_ext")
         nax = int(self.ax_pp_sp.numel())
         rc = L.dfb_pair_tables(p(self.ax_cxyz), p(self.ax_pstart), p(self.ax_nprim), p(self.ax_exp), p(self.ax_coef),
                                p(self.ax_self), p(self.ax_self), p(self.ax_pstart), p(self.ax_pp_sp), 0, nax, 1,
@@ -390,7 +421,8 @@ class DFEngine:
             for l in np.unique(aux.shell_l[s0:s1]):
                 idx = s0 + np.nonzero(aux.shell_l[s0:s1] == l)[0]
                 byl[int(l)] = torch.as_tensor(idx.astype(np.int32), device=self.device)
-            blocks.append((p0, p1, (axb, shifted, byl)))
+            groups = AuxGroups(aux, np.arange(s0, s1), self.device, self.ax_cxyz, shifted, self.ax_atom)
+            blocks.append((p0, p1, (axb, shifted, byl, groups)))
             s0 = s1
         self._aux_blocks, self._aux_blocks_n = blocks, max_naux
         return blocks
@@ -404,41 +436,20 @@ class DFEngine:
         of dropped pairs is the same for every block, so a reused buffer needs
         zeroing once).
         """
-        axb, _shifted, byl = blk
+        axb, _shifted, byl, groups = blk
         nao = self.nao
         X = out if out is not None else torch.empty((p1 - p0, nao, nao), dtype=torch.float64, device=self.device)
-        if self.n_dropped_pairs and not dropped_zero:
-            X.zero_()
-        self._slices_int = self._scratch_slices(False)
-        launches = []
-        seen = set()
-        for la, lb, lc, pairs, _auxs in self.classes3c:
-            if lc not in byl or (la, lb, lc) in seen:
-                continue
-            seen.add((la, lb, lc))
-            auxs = byl[lc]
-            launches.append(self._launch_int(la, lb, lc, self.ps_ao, axb, pairs, auxs, pairs.numel() * auxs.numel(),
-                                             -pairs.numel(), 0, X, (nao * nao, nao, 1), _prec_code(precision)))
-        self._fanout(launches)
+        if not dropped_zero:
+            self._clear_dropped(X, (nao * nao, nao, 1), p1 - p0)
+        self._run_int([self._int3c_work(X, (nao * nao, nao, 1), precision, groups, axb, byl)])
         return X
 
     def deriv3c_block(self, blk, bar: torch.Tensor, grad: torch.Tensor, precision: str = "fp64") -> torch.Tensor:
         """grad += sum over one aux block of bar[P-p0, mu, nu] d(mu nu|P)/dR (block-local adjoint)."""
-        axb, _shifted, byl = blk
+        axb, _shifted, byl, groups = blk
         nao = self.nao
         bar = bar.contiguous()
-        self._slices_der = self._scratch_slices(True)
-        launches = []
-        seen = set()
-        for la, lb, lc, pairs, _auxs in self.classes3c:
-            if lc not in byl or (la, lb, lc) in seen:
-                continue
-            seen.add((la, lb, lc))
-            auxs = byl[lc]
-            launches.append(self._launch_deriv(la, lb, lc, self.ps_ao, axb, pairs, auxs, pairs.numel() * auxs.numel(),
-                                               -pairs.numel(), 0, bar, (nao * nao, nao, 1), grad,
-                                               _prec_code(precision)))
-        self._fanout(launches)
+        self._run_deriv([self._deriv3c_work(bar, (nao * nao, nao, 1), grad, precision, groups, axb, byl)], grad)
         return grad
 
     def _scratch_slices(self, deriv: bool):
@@ -490,9 +501,7 @@ class DFEngine:
         """V[P, Q] = (P|Q), full symmetric (naux, naux)."""
         naux = self.naux
         V = out if out is not None else torch.empty((naux, naux), dtype=torch.float64, device=self.device)
-        self._slices_int = self._scratch_slices(False)
-        self._fanout([self._launch_int(lp, 0, lq, self.ps_aux, self.axs, P, Q, P.numel(), 0, 1, V, (naux, 1, 0))
-                      for lp, lq, P, Q in self.classes2c])
+        self._run_int([self._metric_work(V)])
         # diagonal shell blocks are written from one tile in both orders; make V
         # exactly symmetric as the reference does (cueri_df_cpu.py: V = (V+V^T)/2)
         V.copy_(0.5 * (V + V.T))
@@ -511,12 +520,8 @@ class DFEngine:
         else:
             raise ValueError("layout must be 'Qmn' or 'mnQ'")
         X = out if out is not None else torch.empty(shape, dtype=torch.float64, device=self.device)
-        if self.n_dropped_pairs:
-            X.zero_()
-        self._slices_int = self._scratch_slices(False)
-        pc = _prec_code(precision)
-        self._fanout([self._launch_int(la, lb, lc, self.ps_ao, self.axs, pairs, auxs, pairs.numel() * auxs.numel(),
-                                       -pairs.numel(), 0, X, s, pc) for la, lb, lc, pairs, auxs in self.classes3c])
+        self._clear_dropped(X, s, naux)
+        self._run_int([self._int3c_work(X, s, precision)])
         return X
 
     def deriv3c(self, bar: torch.Tensor, grad: torch.Tensor, layout: str = "Qmn", precision: str = "fp64") -> torch.Tensor:
@@ -529,23 +534,159 @@ class DFEngine:
         else:
             raise ValueError("layout must be 'Qmn' or 'mnQ'")
         bar = bar.contiguous()
-        self._slices_der = self._scratch_slices(True)
-        pc = _prec_code(precision)
-        self._fanout([self._launch_deriv(la, lb, lc, self.ps_ao, self.axs, pairs, auxs, pairs.numel() * auxs.numel(),
-                                         -pairs.numel(), 0, bar, s, grad, pc)
-                      for la, lb, lc, pairs, auxs in self.classes3c])
+        self._run_deriv([self._deriv3c_work(bar, s, grad, precision)], grad)
         return grad
 
     def deriv2c(self, bar: torch.Tensor, grad: torch.Tensor, precision: str = "fp64") -> torch.Tensor:
         """grad += sum_{P,Q} bar[P,Q] d(P|Q)/dR; bar symmetric."""
-        naux = self.naux
         bar = bar.contiguous()
-        self._slices_der = self._scratch_slices(True)
-        pc = _prec_code(precision)
-        self._fanout([self._launch_deriv(lp, 0, lq, self.ps_aux, self.axs, P, Q, P.numel(), 0, 1, bar, (naux, 1, 0),
-                                         grad, pc) for lp, lq, P, Q in self.classes2c])
+        self._run_deriv([self._deriv2c_work(bar, grad, precision)], grad)
         return grad
 
+    # ------------------------------------------------------------ group-kernel routes
+    def _plan(self, kind: str, groups: AuxGroups, precision: str):
+        """Launch plan of one contraction ('int', 'der', or with '2' for the metric) over ``groups``: (ctypes
+        class array, its length, the classes left to the shell-by-shell kernels as (la, lb, lc, pairs)),
+        kept with the groups until the class lists change.
+
+        The group kernels (``dfb_prim_integrals``, ``dfb_grad_contract``) take every class with bra l <= 4
+        (the metric: l <= 8).  Left on ``dfb_rys_*_prec``: AO shells above g, 'mixed_all' (which measures the
+        FP32 shell kernels) and the generic-kernel switch DFB_DISABLE_TMPL."""
+        shells = precision == "mixed_all" or bool(os.environ.get("DFB_DISABLE_TMPL"))
+        f32 = frozenset(mixed_class_table().get("int3c", ())) if precision == "mixed" and kind == "int" else None
+        key = (kind, shells, f32, self._epoch)
+        plan = groups.plans.get(key)
+        if plan is None:
+            if len(groups.plans) > 16:
+                groups.plans.clear()
+            plan = groups.plans[key] = self._make_plan(kind, groups, shells, f32 or ())
+        return plan
+
+    def _make_plan(self, kind: str, groups: AuxGroups, shells: bool, f32):
+        metric, deriv = kind.endswith("2"), kind.startswith("der")
+        if metric:
+            ls = sorted(groups.by_l)
+            classes = [(lp, 0, lq, groups.prim_ids(lp)) for lp in ls for lq in ls if lq <= lp]
+        else:
+            classes = list({(la, lb, lc): (la, lb, lc, pairs) for la, lb, lc, pairs, _a in self._classes3c
+                            if lc in groups.by_l}.values())
+        L = _lib.lib()
+        new = [c for c in classes if not shells and L.dfb_grad_supported(*c[:3], int(metric))]
+        old = [c for c in classes if c not in new]
+        # the longest single tasks (high bra l, few pairs) first: the numerous low classes fill in behind them
+        new.sort(key=lambda c: -(c[0] + c[1]))
+        nprim = {l: hi - lo for l, (lo, hi) in groups.prims.items()}
+        arr = ((_lib.GradClass if deriv else _lib.PrimClass) * max(len(new), 1))()
+        p = _lib.ptr
+        for i, (la, lb, lc, pairs) in enumerate(new):
+            if deriv and not metric:
+                pairs = self._seg_lists[la, lb]
+            n = int(pairs.numel())
+            if deriv:
+                lanes = n * nprim[lc] * ((la + lb + lc + 1) // 2 + 1)
+                nq = 4 if lanes >= GRAD_THREADS else 1
+                chunks = groups.chunks(lc, nq, "after" if metric and la == lc else "all")
+                arr[i] = _lib.GradClass(la, lb, lc, n, p(pairs), p(chunks), chunks.shape[0], nq)
+            else:
+                nq = 1  # a contracted pair's primitives already make a long task
+                chunks = groups.chunks(lc, nq, "own" if metric and la == lc else "all")
+                lst, rows, first = groups.group_rows(lc, nq)
+                ids = groups.group_ids(la) if metric else None
+                arr[i] = _lib.PrimClass(la, lb, lc, n, p(pairs), p(chunks), p(lst), rows.ctypes.data, first.ctypes.data,
+                                        len(rows) - 1, groups.max_shells(lc), p(ids), 0 if ids is None else ids.numel(),
+                                        groups.prims[la][0] if metric else 0, int((la, lb, lc) in f32))
+        per = 0 if deriv or not new else int(L.dfb_prim_scratch(arr, len(new), PRIM_WAVE))
+        return arr, len(new), old, per
+
+    def _int3c_work(self, X, strides, precision, groups=None, axs=None, byl=None):
+        groups, axs, byl = groups or self.groups, axs or self.axs, byl or self.aux_by_l
+        arr, n, old, per = self._plan("int", groups, precision)
+        pc = _prec_code(precision)
+        rest = [(la, lb, lc, self.ps_ao, axs, pairs, byl[lc], pairs.numel() * byl[lc].numel(), -pairs.numel(), 0, X,
+                 strides, pc) for la, lb, lc, pairs in old]
+        return self.bra_ao, groups, arr, n, per, X, strides, rest
+
+    def _clear_dropped(self, X, strides, naux) -> None:
+        """Zeros where the dropped shell pairs would be: their blocks alone, or the whole tensor where they are
+        a quarter of it (a block's rows are short, so its writes cost about four times their bytes)."""
+        lst, sizes, share = self._dropped
+        if not self.n_dropped_pairs:
+            return
+        if share >= 0.25:
+            X.zero_()
+            return
+        rc = _lib.lib().dfb_zero_pairs(ctypes.byref(self.bra_ao), _lib.ptr(lst), lst.numel(), _lib.ptr(sizes), naux,
+                                       _lib.ptr(X), *strides, _stream())
+        _lib.check(rc, "dfb_zero_pairs")
+
+    def _metric_work(self, V):
+        s = (self.naux, 1, 0)
+        arr, n, old, per = self._plan("int2", self.groups, "fp64")
+        left = {c[:3] for c in old}
+        rest = [(lp, 0, lq, self.ps_aux, self.axs, P, Q, P.numel(), 0, 1, V, s)
+                for lp, lq, P, Q in (self.classes2c if old else ()) if (lp, 0, lq) in left]
+        return self.groups.bra, self.groups, arr, n, per, V, s, rest
+
+    def _deriv3c_work(self, bar, strides, grad, precision, groups=None, axs=None, byl=None):
+        groups, axs, byl = groups or self.groups, axs or self.axs, byl or self.aux_by_l
+        arr, n, old, _per = self._plan("der", groups, precision)
+        pc = _prec_code(precision)
+        rest = [(la, lb, lc, self.ps_ao, axs, pairs, byl[lc], pairs.numel() * byl[lc].numel(), -pairs.numel(), 0, bar,
+                 strides, grad, pc) for la, lb, lc, pairs in old]
+        return self.bra_seg, groups, arr, n, bar, strides, rest
+
+    def _deriv2c_work(self, bar, grad, precision):
+        s = (self.naux, 1, 0)
+        arr, n, old, _per = self._plan("der2", self.groups, precision)
+        left = {c[:3] for c in old}
+        pc = _prec_code(precision)
+        rest = [(lp, 0, lq, self.ps_aux, self.axs, P, Q, P.numel(), 0, 1, bar, s, grad, pc)
+                for lp, lq, P, Q in (self.classes2c if old else ()) if (lp, 0, lq) in left]
+        return self.groups.bra, self.groups, arr, n, bar, s, rest
+
+    def _run_int(self, works, then=None):
+        """Run the integral works over the side streams and join.  With a second set ``then`` the current
+        stream waits for the first set only; the fork is returned for ``_join``."""
+        L = _lib.lib()
+        n = max(NSTREAMS, 1)
+        every = works + (then or [])
+        need = max(w[4] for w in every)
+        need = max((need + 31) // 32 * 32 * n, n * 32)
+        if any(w[7] for w in every):
+            need = max(need, self._scratch_for(False, copies=n).numel())
+        buf = self._scratch.get(need, self.device)
+        per = buf.numel() // n // 32 * 32
+        self._slices_int = [buf[i * per:(i + 1) * per] for i in range(n)]
+        fork = self._fork()
+        _main, side, streams = fork
+        for batch in (works, then or []):
+            for bra, groups, arr, ncls, _per, out, (sP, sM, sN), rest in batch:
+                if ncls:
+                    rc = L.dfb_prim_integrals(ctypes.byref(bra), ctypes.byref(groups.c), arr, ncls, _lib.ptr(out), sP, sM,
+                                              sN, _lib.ptr(buf), buf.numel(), streams, len(side))
+                    _lib.check(rc, "dfb_prim_integrals")
+                for i, job in enumerate(rest):
+                    self._launch_int(*job)(int(side[i % n].cuda_stream))
+            if batch is works:
+                self._join(fork)
+        return fork
+
+    def _run_deriv(self, works, grad) -> None:
+        """Run the derivative works over the side streams and join."""
+        L = _lib.lib()
+        n = max(NSTREAMS, 1)
+        if any(w[6] for w in works):
+            self._slices_der = self._scratch_slices(True)
+        fork = self._fork()
+        _main, side, streams = fork
+        for bra, groups, arr, ncls, bar, (sP, sM, sN), rest in works:
+            if ncls:
+                rc = L.dfb_grad_contract(ctypes.byref(bra), ctypes.byref(groups.c), arr, ncls, _lib.ptr(bar), sP, sM, sN,
+                                         _lib.ptr(grad), self.natm, streams, len(side))
+                _lib.check(rc, "dfb_grad_contract")
+            for i, job in enumerate(rest):
+                self._launch_deriv(*job)(int(side[i % n].cuda_stream))
+        self._join(fork)
 
     # ------------------------------------------------------------ overlapped phases of one step
     def metric_cholesky_int3c(self, X: torch.Tensor | None = None, precision: str = "fp64"):
@@ -562,35 +703,11 @@ class DFEngine:
             return V, cholesky_metric(V), self.int3c("Qmn", out=X, precision=precision)
         V = torch.empty((naux, naux), dtype=torch.float64, device=self.device)
         X = X if X is not None else torch.empty((naux, nao, nao), dtype=torch.float64, device=self.device)
-        if self.n_dropped_pairs:
-            X.zero_()
-        self._slices_int = self._scratch_slices(False)
-        first = [self._launch_int(lp, 0, lq, self.ps_aux, self.axs, P, Q, P.numel(), 0, 1, V, (naux, 1, 0))
-                 for lp, lq, P, Q in self.classes2c]
-        pc = _prec_code(precision)
-        second = [self._launch_int(la, lb, lc, self.ps_ao, self.axs, pairs, auxs, pairs.numel() * auxs.numel(),
-                                   -pairs.numel(), 0, X, (nao * nao, nao, 1), pc)
-                  for la, lb, lc, pairs, auxs in self.classes3c]
-        main = torch.cuda.current_stream(self.device)
-        side = self._streams()
-        start = torch.cuda.Event()
-        start.record(main)
-        for st in side:
-            st.wait_event(start)
-        for i, fn in enumerate(first):
-            fn(int(side[i % len(side)].cuda_stream))
-        for st in side:
-            ev = torch.cuda.Event()
-            ev.record(st)
-            main.wait_event(ev)
-        for i, fn in enumerate(second):
-            fn(int(side[(i + len(first)) % len(side)].cuda_stream))
+        self._clear_dropped(X, (nao * nao, nao, 1), naux)
+        fork = self._run_int([self._metric_work(V)], [self._int3c_work(X, (nao * nao, nao, 1), precision)])
         V.copy_(0.5 * (V + V.T))
         L, info = torch.linalg.cholesky_ex(V)
-        for st in side:
-            ev = torch.cuda.Event()
-            ev.record(st)
-            main.wait_event(ev)
+        self._join(fork)
         if int(info.item()) != 0:
             raise RuntimeError(f"metric Cholesky failed (leading minor {int(info.item())} not positive definite)")
         return V, L, X
@@ -598,17 +715,11 @@ class DFEngine:
     def deriv3c_2c(self, bar3: torch.Tensor, bar2: torch.Tensor, grad: torch.Tensor,
                    precision: str = "fp64") -> torch.Tensor:
         """deriv3c(bar3 'Qmn') and deriv2c(bar2) as one fan-out (both add into grad atomically)."""
-        nao, naux = self.nao, self.naux
+        nao = self.nao
         bar3 = bar3.contiguous()
         bar2 = bar2.contiguous()
-        self._slices_der = self._scratch_slices(True)
-        pc = _prec_code(precision)
-        launches = [self._launch_deriv(la, lb, lc, self.ps_ao, self.axs, pairs, auxs, pairs.numel() * auxs.numel(),
-                                       -pairs.numel(), 0, bar3, (nao * nao, nao, 1), grad, pc)
-                    for la, lb, lc, pairs, auxs in self.classes3c]
-        launches += [self._launch_deriv(lp, 0, lq, self.ps_aux, self.axs, P, Q, P.numel(), 0, 1, bar2, (naux, 1, 0),
-                                        grad, pc) for lp, lq, P, Q in self.classes2c]
-        self._fanout(launches)
+        self._run_deriv([self._deriv3c_work(bar3, (nao * nao, nao, 1), grad, precision),
+                         self._deriv2c_work(bar2, grad, precision)], grad)
         return grad
 
 

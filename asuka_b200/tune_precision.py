@@ -86,8 +86,7 @@ def measure(workload: str = "w8") -> dict:
     Eall, gall = _step(eng, Cw, R, X, "mixed_all")
     rows = []
     kinds = [("int3c", (la, lb, lc)) for la, lb, lc, _p, _a in eng.classes3c]
-    kinds += [("deriv3c", (la, lb, lc)) for la, lb, lc, _p, _a in eng.classes3c]
-    kinds += [("deriv2c", (lp, 0, lq)) for lp, lq, _P, _Q in eng.classes2c]
+    # the derivative contractions of the mixed mode run in FP64 (group kernels): nothing to admit
     L = _lib.lib()
     st = int(torch.cuda.current_stream().cuda_stream)
     nao, naux = eng.nao, eng.naux

@@ -190,6 +190,102 @@ int dfb_rys_error(int reset);
 int dfb_gamma_sym(long nP, int nao, int nocc, const double *U, long sU_mu, long sU_P, const double *Cw,
                   double *out, void *stream);
 
+/*
+ * Adjoint-first derivative contraction over shared-exponent auxiliary groups.
+ *
+ * Bra side: AO shell pairs (or parts of one) with the records of their primitive pairs (dfb_pair_ext: p,
+ * 1/p, 2 pi^(5/2) cK / p, P, 2a, 2b), or (b_dummy = 1, the metric) one primitive aux function per
+ * entry: shA = its representative shell, shB = its group, P = its centre whatever the record says.
+ */
+typedef struct {
+    const int *shA, *shB, *pstart, *npair;
+    const double *rec;             /* 8 doubles per primitive pair, 16-byte aligned */
+    const double *cxyz;
+    const int *aostart, *atom;
+    int b_dummy;
+} dfb_bra_t;
+
+/*
+ * Groups of aux shells with one centre, angular momentum and exponent list.  info holds 6 ints per
+ * group: representative shell, first primitive, primitives, shells, first coefficient
+ * (coef[first + s * primitives + k]), first entry of the shell list.
+ */
+typedef struct {
+    const int *info;
+    const double *coef;
+    const int *shells;
+    const double *pexp, *rexp;
+    const double *cxyz;
+    const int *aostart, *atom;
+} dfb_groups_t;
+
+/*
+ * One angular class: bra entries (device list) x chunks of at most nq group primitives (device, 5
+ * ints each: group, first primitive, count, first row, first bra entry to use).
+ */
+typedef struct {
+    int la, lb, lc, npair;
+    const int *pairs;
+    const int *chunks;
+    int nchunk, nq;
+} dfb_grad_class_t;
+
+/* Order the side streams after `main` (fork), or `main` after the side streams (join). */
+int dfb_fork(void *main_stream, void *const *streams, int nstreams);
+int dfb_join(void *main_stream, void *const *streams, int nstreams);
+
+int dfb_pair_ext(const double *eta, const double *Px, const double *Py, const double *Pz, const double *cK,
+                 const double *ea, const double *eb, long npp, double *rec, void *stream);
+
+/* 1 when dfb_grad_contract takes the class (bra l <= 4; metric bra l <= 8; aux l <= 8). */
+int dfb_grad_supported(int la, int lb, int lc, int b_dummy);
+
+/*
+ * grad (natm, 3) += sum bar . d(mu nu|P)/dR (AO bra) or sum bar . d(P|Q)/dR (metric bra, over the
+ * unordered pairs listed, counted twice) for symmetric bar at bar[P*sP + mu*sM + nu*sN] (metric:
+ * bar[P*sP + Q*sM]).  Class i runs on streams[i % nstreams]; the caller orders the streams.  FP64.  Replaces df_int3c2e_deriv_contracted_cart_allsp_atomgrad_inplace_device
+ * and its metric analogue (asuka/integrals/grad.py:537-565,659-687).
+ */
+int dfb_grad_contract(const dfb_bra_t *bra, const dfb_groups_t *groups, const dfb_grad_class_t *cls, int ncls,
+                      const double *bar, long sP, long sM, long sN, double *grad, int natm,
+                      void *const *streams, int nstreams);
+
+/*
+ * Integral counterpart: one angular class of 3c integrals (AO bra) or of the metric (metric bra).
+ * chunks as in dfb_grad_class_t; groups (device): (group, first row) per group of the class;
+ * rows, first_chunk (host, ngroup + 1): per group the first row and the first chunk.  Metric only:
+ * bra_groups (device) the groups of the bra l, bra_prim0 their first primitive.
+ */
+typedef struct {
+    int la, lb, lc, npair;
+    const int *pairs;
+    const int *chunks;
+    const int *groups;
+    const long *rows, *first_chunk;
+    int ngroup, max_shells;        /* largest shell count of a listed group */
+    const int *bra_groups;
+    int nbra_groups, bra_prim0;
+    int f32;                       /* 1: FP32 recurrence tables and accumulators per primitive (AO bra) */
+} dfb_prim_class_t;
+
+long dfb_prim_scratch(const dfb_prim_class_t *cls, int ncls, long target);
+
+/*
+ * out[P*sP + mu*sM + nu*sN] = (mu nu|P), both orders of (mu, nu) (AO bra), or out[P*sP + Q*sM] = (P|Q),
+ * both orders (metric bra), for every listed class, evaluated once per primitive of a group.  Class i
+ * runs on streams[i % nstreams] with its own slice of scratch; the caller orders the streams.  FP64; classes with f32 set evaluate each primitive with FP32 tables and
+ * accumulators where the register kernel takes them (roots, weights and the contraction stay FP64).
+ * Replaces df_int3c2e_rys_device_block + scatter and df_metric_2c2e_rys_device
+ * (asuka/cueri/gpu.py:2742,2104).
+ */
+int dfb_prim_integrals(const dfb_bra_t *bra, const dfb_groups_t *groups, const dfb_prim_class_t *cls, int ncls,
+                       double *out, long sP, long sM, long sN, double *scratch, long scratch_doubles,
+                       void *const *streams, int nstreams);
+
+/* out = 0 in both orders for the listed AO pairs (device list; shell_size = functions per AO shell). */
+int dfb_zero_pairs(const dfb_bra_t *bra, const int *list, int npairs, const int *shell_size, long naux, double *out,
+                   long sP, long sM, long sN, void *stream);
+
 /* Scratch doubles dfb_rys_int / dfb_rys_deriv need for this class and task count. */
 long dfb_rys_scratch_doubles(int la, int lb, int lc, long ntask, int deriv);
 
