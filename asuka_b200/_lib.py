@@ -97,6 +97,8 @@ _SIGS = {
                                           ctypes.c_long, ctypes.POINTER(ctypes.c_void_p), ctypes.c_int]),
     "dfb_zero_pairs": (ctypes.c_int, [ctypes.POINTER(Bra), _d, ctypes.c_int, _d, ctypes.c_long, _d, ctypes.c_long,
                                       ctypes.c_long, ctypes.c_long, _d]),
+    "dfb_dsyrk": (ctypes.c_int, [ctypes.c_int, ctypes.c_long, ctypes.c_long, _d, ctypes.c_long, ctypes.c_long, _d,
+                                 ctypes.c_long, _d]),
     "dfb_launch_count": (ctypes.c_long, []),
     "dfb_rys_scratch_doubles": (ctypes.c_long, [ctypes.c_int] * 3 + [ctypes.c_long, ctypes.c_int]),
     "dfb_fp64_fma_probe": (ctypes.c_int, [_d, ctypes.c_int, ctypes.c_int, ctypes.c_int, _d]),

@@ -142,12 +142,10 @@ class BatchedDFJK:
         W3 = Y.view(naux, nao, nocc)
         K = m.K
         K.zero_()
-        qb = max(1, (1 << 27) // max(nao * nocc, 1))
         if mixed:
             _tc.syrk_qblocks(W3, out=K)  # split-BF16 tcgen05 update, W read in place
-        for q0 in range(0, 0 if mixed else naux, qb):
-            Wc = W3[q0:q0 + qb].permute(1, 0, 2).reshape(nao, -1)
-            K.addmm_(Wc, Wc.T)
+        else:
+            _la.exchange_update(W3, K)
         K.copy_(0.5 * (K + K.T))
         J = m.J
         J.zero_()

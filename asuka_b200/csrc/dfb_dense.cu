@@ -1,4 +1,6 @@
-// FP64 dense kernel of the DF gradient: the 3c adjoint
+// FP64 dense kernels: the 3c adjoint of the DF gradient, and the exchange update (k_dsyrk).
+//
+// The 3c adjoint
 //
 //   Gamma[P] = Cw A_P Cw^T = U_P Cw^T,    U_P = Cw A_P,   A_P = d_P I - Z_P / 2 (symmetric)
 //
@@ -124,6 +126,94 @@ __global__ void __launch_bounds__(NT, 3) k_gamma_sym(long nP, int nao, int nocc,
     }
 }
 
+// Exchange update K += sum_k A(m, k) A(n, k) of the FP64 path, A(m, k) = W[kq * skq + m * sm + k1] with
+// k = kq * nk1 + k1 (W[Q, mu, i]: skq = nao nocc, sm = nocc, nk1 = nocc), so W is read in place.
+// FP64-FMA-bound.  Only the 64 x 64 tiles on and above the diagonal are formed (0.57 of a full product at
+// nao 416) and k is cut into spans over blockIdx.y, so that a few hundred columns still fill the chip;
+// the spans add into K atomically, off-diagonal tiles in both orders.  128 threads, 8 x 4 outputs each
+// (12 shared-memory reads per 32 multiply-adds), k chunks of 16 double-buffered through registers.
+constexpr int ST = 64;        // tile edge
+constexpr int SKC = 16;       // k per chunk
+constexpr int SNT = 128;      // threads
+constexpr int SP = ST + 1;    // row stride of a chunk: the transposing stores of a half warp hit 16 banks
+
+__global__ void __launch_bounds__(SNT, 4) k_dsyrk(int n, long K, long nk1, const double* __restrict__ W, long skq, long sm,
+                                               double* __restrict__ C, long ldc, long kspan, int T) {
+    __shared__ double sA[2][SKC * SP], sB[2][SKC * SP];
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    int idx = blockIdx.x, mt = 0;
+    while (idx >= T - mt) {
+        idx -= T - mt;
+        ++mt;
+    }
+    const int nt = mt + idx, m0 = mt * ST, n0 = nt * ST;
+    const bool diag = mt == nt;
+    const long kbeg = (long)blockIdx.y * kspan, kend = kbeg + kspan < K ? kbeg + kspan : K;
+    const int lk = tid & (SKC - 1), lr = tid >> 4;  // this thread loads column lk of rows lr + 8 i
+    double va[8], vb[8];
+    auto load = [&](long k0) {
+        const long k = k0 + lk;
+        const bool in = k < kend;
+        const long kq = in ? k / nk1 : 0;
+        const double* p = W + kq * skq + (in ? k - kq * nk1 : 0);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int r = lr + 8 * i;
+            va[i] = (in && m0 + r < n) ? __ldg(p + (long)(m0 + r) * sm) : 0.0;
+            if (!diag) vb[i] = (in && n0 + r < n) ? __ldg(p + (long)(n0 + r) * sm) : 0.0;
+        }
+    };
+    auto store = [&](int buf) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            sA[buf][lk * SP + lr + 8 * i] = va[i];
+            if (!diag) sB[buf][lk * SP + lr + 8 * i] = vb[i];
+        }
+    };
+    double acc[8][4];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0.0;
+    load(kbeg);
+    store(0);
+    __syncthreads();
+    int buf = 0;
+    for (long k0 = kbeg; k0 < kend; k0 += SKC) {
+        const bool more = k0 + SKC < kend;
+        if (more) load(k0 + SKC);
+        const double* pa = sA[buf] + 8 * ty;
+        const double* pb = (diag ? sA[buf] : sB[buf]) + tx;
+#pragma unroll
+        for (int c = 0; c < SKC; ++c) {
+            double a[8], b[4];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) a[i] = pa[c * SP + i];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) b[j] = pb[c * SP + 16 * j];
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
+        }
+        if (more) store(buf ^ 1);
+        __syncthreads();
+        buf ^= 1;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int m = m0 + 8 * ty + i;
+        if (m >= n) continue;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int c = n0 + tx + 16 * j;
+            if (c >= n || (diag && c < m)) continue;  // a diagonal tile mirrors its upper part
+            atomicAdd(C + (long)m * ldc + c, acc[i][j]);
+            if (c != m) atomicAdd(C + (long)c * ldc + m, acc[i][j]);
+        }
+    }
+}
+
 }  // namespace dense
 }  // namespace dfb
 
@@ -153,5 +243,30 @@ extern "C" int dfb_gamma_sym(long nP, int nao, int nocc, const double* U, long s
     count_launches(1);
     e = cudaGetLastError();
     if (e != cudaSuccess) return set_cuda_error("k_gamma_sym launch", e);
+    return DFB_OK;
+}
+
+extern "C" int dfb_dsyrk(int n, long nkq, long nk1, const double* W, long skq, long sm, double* C, long ldc, void* stream) {
+    clear_error();
+    if (n < 0 || nkq < 0 || nk1 < 0 || ldc < n)
+        return set_error(DFB_ERR_INVALID, "invalid sizes to dfb_dsyrk (n %d, k %ld x %ld)", n, nkq, nk1);
+    const long K = nkq * nk1;
+    if (n == 0 || K == 0) return DFB_OK;
+    if (!W || !C) return set_error(DFB_ERR_INVALID, "invalid pointers to dfb_dsyrk");
+    const int T = (n + dense::ST - 1) / dense::ST;
+    const long ntiles = (long)T * (T + 1) / 2;
+    if (ntiles > 0x7fffffffL) return set_error(DFB_ERR_UNSUPPORTED, "n %d too large", n);
+    // spans: about four resident blocks per SM, each at least 512 long (a span ends in 64 x 64 atomic additions)
+    long ns = (4 * 148 + ntiles - 1) / ntiles;
+    if (ns > (K + 511) / 512) ns = (K + 511) / 512;
+    if (ns < 1) ns = 1;
+    long span = (K + ns - 1) / ns;
+    span = (span + dense::SKC - 1) / dense::SKC * dense::SKC;
+    ns = (K + span - 1) / span;
+    dense::k_dsyrk<<<dim3((unsigned)ntiles, (unsigned)ns), dense::SNT, 0, (cudaStream_t)stream>>>(n, K, nk1, W, skq, sm, C,
+                                                                                                  ldc, span, T);
+    count_launches(1);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return set_cuda_error("k_dsyrk launch", e);
     return DFB_OK;
 }

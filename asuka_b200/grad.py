@@ -148,8 +148,7 @@ def df_contract(engine: DFEngine, Cw: torch.Tensor, X: torch.Tensor, L: torch.Te
         if mixed and MIXED_K_TC:
             K = _tc.syrk_qblocks(W3)
         else:
-            W2 = W3.permute(1, 0, 2).reshape(nao, naux * nocc)
-            K = W2 @ W2.T
+            K = _la.exchange_update(W3, torch.zeros((nao, nao), dtype=W3.dtype, device=W3.device))
         K = 0.5 * (K + K.T)
     E = 0.5 * torch.dot(rho, d) - 0.25 * torch.sum(M * M)
     saved = dict(X=X, L=L, d=d, W=W, M=M, D=D, Linv_blocks=Linv_blocks)
@@ -289,9 +288,8 @@ def df_energy_grad_streamed(engine: DFEngine, Cw: torch.Tensor, aux_block: int =
     qb = max(1, (1 << 27) // max(nao * nocc, 1))
     if precision != "fp64":
         _tc.syrk_qblocks(W3, out=K)  # reads W in place, k = (Q, i)
-    for q0 in range(0, naux if precision == "fp64" else 0, qb):
-        Wc = W3[q0:q0 + qb].permute(1, 0, 2).reshape(nao, -1)
-        K.addmm_(Wc, Wc.T)
+    else:
+        _la.exchange_update(W3, K)
     K = 0.5 * (K + K.T)
     D = Cw @ Cw.T
     E = 0.5 * torch.dot(rho, d) - 0.25 * torch.sum(D * K)

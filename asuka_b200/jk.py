@@ -22,7 +22,10 @@ from __future__ import annotations
 
 import torch
 
+from . import linalg as _la
 from . import tc as _tc
+
+HALF_ELEMS = 1 << 25  # elements of the half-transformed block U a J/K build keeps at least (268 MB)
 
 
 def _sym(A: torch.Tensor) -> torch.Tensor:
@@ -42,13 +45,14 @@ def df_K_from_BQ_Cw(BQ: torch.Tensor, Cw: torch.Tensor, q_block: int = 256, prec
     K = torch.zeros((nao, nao), dtype=torch.float64, device=BQ.device)
     if nocc == 0:
         return K
-    for q0 in range(0, naux, q_block):
-        q1 = min(naux, q0 + q_block)
+    # q_block bounds the caller's memory; blocks below HALF_ELEMS are run together (fewer, fuller products)
+    step = max(q_block, min(naux, HALF_ELEMS // max(nao * nocc, 1)))
+    for q0 in range(0, naux, step):
+        q1 = min(naux, q0 + step)
         blk = BQ[q0:q1]
         if precision == "fp64":
             U = torch.matmul(blk.reshape(-1, nao), Cw).reshape(q1 - q0, nao, nocc)
-            U2 = U.permute(1, 0, 2).reshape(nao, -1)
-            K += U2 @ U2.T
+            _la.exchange_update(U, K)
         else:
             U = _tc.matmul(blk.reshape(-1, nao), Cw).view(q1 - q0, nao, nocc)
             _tc.syrk_qblocks(U, out=K)

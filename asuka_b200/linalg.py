@@ -15,6 +15,8 @@ from __future__ import annotations
 
 import torch
 
+from . import _lib
+
 NB = 256  # rows per diagonal block
 
 
@@ -104,3 +106,19 @@ def solve_lower_right_T(L: torch.Tensor, X: torch.Tensor, inv: list[torch.Tensor
         rhs = X[:, r0:r1] if r0 == 0 else torch.addmm(X[:, r0:r1], B[:, :r0], L[r0:r1, :r0].T, alpha=-1.0)
         B[:, r0:r1] = rhs @ inv[i].T
     return B
+
+
+def exchange_update(W: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
+    """out += sum_Q W_Q W_Q^T for W (naux, nao, nocc) FP64, in place and without a transposed copy of W.
+
+    On the GPU the library's symmetric kernel (``dfb_dsyrk``: half the multiply-adds of a full product, k
+    split over the chip); its two triangles differ by the rounding of their span sums."""
+    naux, nao, nocc = W.shape
+    if not W.is_cuda:
+        W2 = W.permute(1, 0, 2).reshape(nao, naux * nocc)
+        return out.addmm_(W2, W2.T)
+    W = W.contiguous()
+    rc = _lib.lib().dfb_dsyrk(nao, naux, nocc, _lib.ptr(W), nao * nocc, nocc, _lib.ptr(out), out.stride(0),
+                              int(torch.cuda.current_stream(W.device).cuda_stream))
+    _lib.check(rc, "dfb_dsyrk")
+    return out

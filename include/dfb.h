@@ -282,6 +282,13 @@ int dfb_prim_integrals(const dfb_bra_t *bra, const dfb_groups_t *groups, const d
                        double *out, long sP, long sM, long sN, double *scratch, long scratch_doubles,
                        void *const *streams, int nstreams);
 
+/*
+ * FP64 exchange update C[m*ldc + n] += sum_k A(m, k) A(n, k), A(m, k) = W[(k / nk1)*skq + m*sm + k % nk1]
+ * with k < nkq*nk1 (W[Q, mu, i]: skq = nao*nocc, sm = nocc, nk1 = nocc).  Adds with FP64 atomics, both
+ * orders.  Replaces the cuBLAS products of hf_df_jk_cuda_ext.cpp:231-598 in FP64.
+ */
+int dfb_dsyrk(int n, long nkq, long nk1, const double *W, long skq, long sm, double *C, long ldc, void *stream);
+
 /* out = 0 in both orders for the listed AO pairs (device list; shell_size = functions per AO shell). */
 int dfb_zero_pairs(const dfb_bra_t *bra, const int *list, int npairs, const int *shell_size, long naux, double *out,
                    long sP, long sM, long sN, void *stream);
