@@ -40,8 +40,11 @@ _TABLE_READY: set[int] = set()
 PRIM_SCREEN = 1e-20  # primitive-pair magnitude bound below which a pair is skipped (0 = evaluate all)
 NSTREAMS = int(os.environ.get("DFB_STREAMS", "8"))  # side streams for per-class launches (2/4/6/8 measured: 8 fastest)
 PRIM_WAVE = 1 << 23  # doubles of primitive integrals per stream and wave of a class (64 MB)
-GRAD_THREADS = 1 << 19  # lanes of one derivative class below which its tasks are single primitives
-SEG_PRIMS = 4  # primitive pairs of a derivative task: contracted pairs are cut, so that no task outlasts the rest
+# Lanes of one derivative class from which its tasks take 4 and 16 primitives: a task's set-up (rows, pair data,
+# closing sums) is shared, but too few tasks leave SMs idle (2^19 and none: (H2O)8 7.15 ms, decane 2.92;
+# 2^17 and 2^20: 6.51 and 2.48)
+GRAD_THREADS, GRAD_BIG = 1 << 17, 1 << 20
+SEG_PRIMS = 8  # primitive pairs of a derivative task: contracted pairs are cut, so that no task outlasts the rest
 NROOTS_SLOTS = 11  # DFB_NROOTS_MAX + 1
 _SIDE_STREAMS: dict[int, list] = {}
 
@@ -584,7 +587,7 @@ class DFEngine:
             n = int(pairs.numel())
             if deriv:
                 lanes = n * nprim[lc] * ((la + lb + lc + 1) // 2 + 1)
-                nq = 4 if lanes >= GRAD_THREADS else 1
+                nq = 16 if lanes >= GRAD_BIG else 4 if lanes >= GRAD_THREADS else 1
                 chunks = groups.chunks(lc, nq, "after" if metric and la == lc else "all")
                 arr[i] = _lib.GradClass(la, lb, lc, n, p(pairs), p(chunks), chunks.shape[0], nq)
             else:
