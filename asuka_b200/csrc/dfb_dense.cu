@@ -214,6 +214,81 @@ __global__ void __launch_bounds__(SNT, 4) k_dsyrk(int n, long K, long nk1, const
     }
 }
 
+// Inverses of the nb x nb diagonal blocks of a lower-triangular L by forward substitution.  A CTA takes 32
+// columns of one block (lane = column) and walks its rows in panels of 16, the next panel of L read ahead
+// through registers: each warp forms the dot products of two rows with the solved ones, then one warp solves
+// the panel's triangle.  Bound by the chain of panels, not by the number of blocks, and one launch where
+// batched library solves and products of growing blocks took twenty.
+constexpr int IC = 32, IW = 8, INB = 256, IP = 16;
+
+__global__ void __launch_bounds__(32 * IW) k_tri_inv(int n, int nb, const double* __restrict__ L, long ldl,
+                                                     double* __restrict__ out) {
+    extern __shared__ double sm[];
+    double* x = sm;                       // [nb][32] solved rows
+    double* S = x + (long)nb * IC;        // [IP][32]
+    double* pan = S + IP * IC;            // [2][IP][nb]: rows of the panel, columns from j0
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int r0 = blockIdx.y * nb, m = n - r0 < nb ? n - r0 : nb;  // rows of this block
+    const int j0 = blockIdx.x * IC, col = j0 + lane;
+    const double* Lb = L + (long)r0 * ldl + r0;
+    double* O = out + (long)blockIdx.y * nb * nb;
+    if (j0 >= m) return;
+    for (int i = w; i < j0; i += IW) O[(long)i * nb + col] = 0.0;  // above the diagonal (col < nb)
+    double pre[IP];  // this thread's column j0 + tid of the next panel's rows
+    auto fetch = [&](int p0) {
+#pragma unroll
+        for (int r = 0; r < IP; ++r) {
+            const int i = p0 + r, k = j0 + tid;
+            pre[r] = (i < m && k <= i) ? __ldg(Lb + (long)i * ldl + k) : 0.0;
+        }
+    };
+    auto put = [&](int buf) {
+        if (tid < nb - j0) {
+#pragma unroll
+            for (int r = 0; r < IP; ++r) pan[(buf * IP + r) * nb + tid] = pre[r];
+        }
+    };
+    fetch(j0);
+    put(0);
+    __syncthreads();
+    int buf = 0;
+    for (int p0 = j0; p0 < m; p0 += IP, buf ^= 1) {
+        const bool more = p0 + IP < m;
+        if (more) fetch(p0 + IP);
+        const double* P = pan + buf * IP * nb;
+#pragma unroll
+        for (int h = 0; h < IP / IW; ++h) {
+            const double* row = P + (w + h * IW) * nb;
+            double s[4] = {0.0, 0.0, 0.0, 0.0};
+            for (int k = 0; k < p0 - j0; k += 4) {  // p0 - j0 is a multiple of IP
+#pragma unroll
+                for (int q = 0; q < 4; ++q) s[q] = fma(row[k + q], x[(j0 + k + q) * IC + lane], s[q]);
+            }
+            S[(w + h * IW) * IC + lane] = (s[0] + s[1]) + (s[2] + s[3]);
+        }
+        __syncthreads();
+        if (w == 0) {
+            double xr[IP];
+#pragma unroll
+            for (int r = 0; r < IP; ++r) {
+                const int i = p0 + r;
+                double t = (col == i ? 1.0 : 0.0) - S[r * IC + lane];
+#pragma unroll
+                for (int q = 0; q < IP; ++q)
+                    if (q < r) t = fma(-P[r * nb + p0 - j0 + q], xr[q], t);
+                const double d = P[r * nb + p0 - j0 + r];
+                xr[r] = (i < m && col <= i) ? t / d : 0.0;
+                if (i < m) {
+                    x[i * IC + lane] = xr[r];
+                    if (col < m) O[(long)i * nb + col] = xr[r];
+                }
+            }
+        }
+        if (more) put(buf ^ 1);
+        __syncthreads();
+    }
+}
+
 }  // namespace dense
 }  // namespace dfb
 
@@ -269,4 +344,20 @@ extern "C" int dfb_dsyrk(int n, long nkq, long nk1, const double* W, long skq, l
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return set_cuda_error("k_dsyrk launch", e);
     return DFB_OK;
+}
+
+extern "C" int dfb_tri_inv(int n, int nb, const double* L, long ldl, double* out, void* stream) {
+    clear_error();
+    if (n < 0 || nb < 32 || nb > dense::INB || nb % 32 || ldl < n)
+        return set_error(DFB_ERR_INVALID, "invalid sizes to dfb_tri_inv (n %d, nb %d)", n, nb);
+    if (n == 0) return DFB_OK;
+    if (!L || !out) return set_error(DFB_ERR_INVALID, "invalid pointers to dfb_tri_inv");
+    const int nblk = (n + nb - 1) / nb;
+    const size_t sm = sizeof(double) * ((size_t)nb * dense::IC + dense::IP * dense::IC + 2 * dense::IP * nb);
+    cudaError_t e = cudaFuncSetAttribute(dense::k_tri_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e != cudaSuccess) return set_cuda_error("cudaFuncSetAttribute(k_tri_inv)", e);
+    dense::k_tri_inv<<<dim3(nb / dense::IC, nblk), 32 * dense::IW, sm, (cudaStream_t)stream>>>(n, nb, L, ldl, out);
+    count_launches(1);
+    e = cudaGetLastError();
+    return e == cudaSuccess ? DFB_OK : set_cuda_error("k_tri_inv launch", e);
 }

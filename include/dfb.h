@@ -289,6 +289,13 @@ int dfb_prim_integrals(const dfb_bra_t *bra, const dfb_groups_t *groups, const d
  */
 int dfb_dsyrk(int n, long nkq, long nk1, const double *W, long skq, long sm, double *C, long ldc, void *stream);
 
+/*
+ * Inverses of the nb x nb diagonal blocks (the last one may be smaller) of the lower-triangular L (n, n) with
+ * row stride ldl: block b row-major at out + b*nb*nb with row stride nb.  nb a multiple of 32, at most 256;
+ * entries beyond a smaller last block are not written.
+ */
+int dfb_tri_inv(int n, int nb, const double *L, long ldl, double *out, void *stream);
+
 /* out = 0 in both orders for the listed AO pairs (device list; shell_size = functions per AO shell). */
 int dfb_zero_pairs(const dfb_bra_t *bra, const int *list, int npairs, const int *shell_size, long naux, double *out,
                    long sP, long sM, long sN, void *stream);

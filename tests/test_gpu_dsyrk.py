@@ -37,3 +37,24 @@ def test_exchange_update_rejects_bad_sizes():
     assert L.dfb_dsyrk(4, 2, 3, 0, 12, 3, 0, 4, None) == -1   # no pointers
     assert L.dfb_dsyrk(4, 2, 3, 0, 12, 3, 0, 3, None) == -1   # ldc < n
     assert L.dfb_dsyrk(0, 2, 3, 0, 12, 3, 0, 0, None) == 0    # nothing to do
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 64, 255, 256, 257, 300, 520])
+@pytest.mark.parametrize("nb", [32, 96, 256])
+def test_diag_block_inverses(n, nb):
+    """Block inverses by forward substitution (``dfb_tri_inv``), row- and column-major factors: the residual of
+    a substitution is within n ulp of the magnitudes of L times its inverse."""
+    from asuka_b200.linalg import diag_block_inverses
+
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n)
+    A = torch.randn((n, n + 8), generator=g, dtype=torch.float64, device="cuda")
+    L = torch.linalg.cholesky(A @ A.T + n * torch.eye(n, dtype=torch.float64, device="cuda"))
+    for F in (L.contiguous(), L.T.contiguous().T):
+        for i, inv in enumerate(diag_block_inverses(F, nb)):
+            r0 = i * nb
+            blk = L[r0:r0 + nb, r0:r0 + nb]
+            eye = torch.eye(blk.shape[0], dtype=L.dtype, device="cuda")
+            bound = nb * 2.3e-16 * float((blk.abs() @ inv.abs()).max())
+            assert float((blk @ inv - eye).abs().max()) <= bound
+            assert float(torch.triu(inv, 1).abs().max()) == 0.0 if inv.shape[0] > 1 else True
