@@ -68,9 +68,16 @@ def _deriv3c_traffic():
     return None, None
 
 
+def _distinct_prims(aux, l) -> float:
+    """Distinct (centre, exponent) pairs among the aux shells of angular momentum l: the primitive functions the
+    contracted shells are combinations of, each of which the group kernels evaluate once."""
+    return float(len({(int(aux.shell_atom[s]), float(e)) for s in np.nonzero(aux.shell_l == l)[0]
+                      for e in aux.prim_exp[aux.shell_prim_start[s]:aux.shell_prim_start[s] + aux.shell_nprim[s]]}))
+
+
 def flops_3c(ao, aux, deriv: bool = False) -> float:
     """Algorithmic FLOPs of the 3c integrals (deriv=False) or of the 3c derivative contraction,
-    summed over every (AO shell pair, aux shell) triplet with the per-unit model
+    summed over every AO shell pair and distinct aux primitive (K_P: their count) with the per-unit model
     K_ab K_P n_r (3 n_A n_B n_P + 9 (l_a+l_b+1)(l_P+1)) for integrals and
     K_ab K_P n_r' (25 n_A n_B n_P + 9 (l_a+l_b+2)(l_P+2)) for the derivative."""
     if deriv:
@@ -82,7 +89,7 @@ def flops_3c(ao, aux, deriv: bool = False) -> float:
     lb = ao.shell_l[sp.sp_B]
     tot = 0.0
     for lp in np.unique(aux.shell_l):
-        kp = float(aux.shell_nprim[aux.shell_l == lp].sum())
+        kp = _distinct_prims(aux, lp)
         for a in np.unique(la):
             for b in np.unique(lb):
                 m = (la == a) & (lb == b)
@@ -97,7 +104,7 @@ def flops_3c(ao, aux, deriv: bool = False) -> float:
 
 def flops_deriv3c(ao, aux) -> float:
     """Algorithmic FLOPs of the 3c derivative contraction, per primitive triplet
-    K_ab K_P n_r' (25 n_A n_B n_P + 9 (l_a+l_b+2)(l_P+2)) summed over every (AO shell pair, aux shell)."""
+    K_ab K_P n_r' (25 n_A n_B n_P + 9 (l_a+l_b+2)(l_P+2)) summed over every AO shell pair and distinct aux primitive."""
     from asuka_b200.basis import build_shell_pairs_l_order, ncart
 
     sp = build_shell_pairs_l_order(ao)
@@ -105,7 +112,7 @@ def flops_deriv3c(ao, aux) -> float:
     lb = ao.shell_l[sp.sp_B]
     tot = 0.0
     for lp in np.unique(aux.shell_l):
-        kp = float(aux.shell_nprim[aux.shell_l == lp].sum())
+        kp = _distinct_prims(aux, lp)
         for a in np.unique(la):
             for b in np.unique(lb):
                 m = (la == a) & (lb == b)
@@ -402,7 +409,7 @@ def run_gpu(args) -> dict | None:
 
     traffic, traffic_src = _deriv3c_traffic()
     tab = dfmod.mixed_class_table()
-    mixed_counts = ", ".join(f"{len(tab.get(k, ()))} {k}" for k in ("int3c", "deriv3c", "deriv2c"))
+    mixed_counts = f"{len(tab.get('int3c', ()))} int3c"
     ms_mx, clk = results["mixed"]
     ms_64, clk64 = results["fp64"]
     out = {
@@ -412,7 +419,7 @@ def run_gpu(args) -> dict | None:
         "config": {"workload": WORKLOAD, "nao": nao, "naux": naux,
                    "precision": "mixed: FP32-component Rys kernels for the angular classes the precision table admits "
                                 f"({mixed_counts}, chosen by asuka_b200.tune_precision within 2.5e-7 Eh and 2.5e-7 "
-                                "Eh/bohr), split-BF16 tcgen05 exchange update; FP64 roots/weights, metric, solves, "
+                                "Eh/bohr), split-BF16 tcgen05 exchange update; FP64 roots/weights, metric, solves, derivative contractions, "
                                 "Y = X Cw, adjoints, energy and gradient accumulation",
                    "l2": "working set (3c tensor 2.5 GB) > L2 126 MB", "replicas": world if world > 1 else None},
         "fp64_ms_per_step": round(ms_64, 4),
@@ -424,7 +431,7 @@ def run_gpu(args) -> dict | None:
                 "d2h_bytes_per_step": int(gh.numel() * 8 + 8)},
         "gpu_launches": launches["mixed"],
         "gpu_launches_fp64_run": launches["fp64"],
-        "roofline": {"kernel": "k_rys<DERIV> (3c derivative contraction, all classes)", "bound": "fp64",
+        "roofline": {"kernel": "k_rys_grad (3c derivative contraction, all classes)", "bound": "fp64",
                      "achieved": round(achieved, 3), "peak": fp64_peak, "unit": "TFLOP/s",
                      "frac": round(achieved / fp64_peak, 4), "peak_source": fp64_src,
                      "fp64_dgemm_tflops": round(dgemm_peak, 2),
