@@ -825,8 +825,6 @@ struct GradLaunch {
 };
 
 // Shared memory: gradient, then per warp the rows of qc primitives (prim doubles each) and extra doubles.
-constexpr int GRAD_CARVE = 44;  // percent of the SM's 228 KB
-constexpr size_t GRAD_CARVE_BYTES = 48 * 1024;
 template <class K>
 inline cudaError_t grad_launch(K kern, const GradLaunch& L, int qc, int prim, int extra, int ny) {
     GradArgs g = L.g;
@@ -836,12 +834,6 @@ inline cudaError_t grad_launch(K kern, const GradLaunch& L, int qc, int prim, in
     const size_t sm = sizeof(double) * ((g.smem_grad ? 3 * g.natm : 0) + (size_t)GRAD_WARPS * g.warp_sz);
     if (sm > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e != cudaSuccess) return e;
-    }
-    // one carve-out for every class: an SM drains before it changes its split of shared memory and L1, which
-    // would serialise classes that run side by side on the streams
-    if (sm <= GRAD_CARVE_BYTES) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, GRAD_CARVE);
         if (e != cudaSuccess) return e;
     }
     // tiles of pairs waste the end of the last tile: worth it from two tiles on
