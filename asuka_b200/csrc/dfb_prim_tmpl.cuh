@@ -3,7 +3,11 @@
 // The auxiliary shells of a group are contractions of one primitive set, so (e 0|f) is evaluated
 // once per (AO pair, primitive) into the rows of W (tiles of 32 pairs, 256-byte segments), and
 // k_prim_out contracts a group's rows to its shells, applies the horizontal recurrence and writes
-// the 3c tensor (k_prim_out2: both sides of the metric).  The rows of a wave stay in L2.
+// the 3c tensor (k_prim_out2: both sides of the metric).  Rows of up to 64 MB per stream and wave.
+//
+// (H2O)8/ma-TZVP, 416 AO / 1824 aux: 3c integrals 5.5 ms with one evaluation per shell, 4.75 ms here, of which
+// the contraction k_prim_out takes most (its blocks wait on dependent loads); metric 0.80 -> 0.33 ms.
+// (H2O)3/ma-QZVP, whole FP64 step: 52.7 -> 31.8 ms.
 #pragma once
 #include "dfb_grad_tmpl.cuh"
 
