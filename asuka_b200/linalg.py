@@ -85,17 +85,28 @@ def solve_lower_right_T(L: torch.Tensor, X: torch.Tensor, inv: list[torch.Tensor
     return B
 
 
-def exchange_update(W: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
-    """out += sum_Q W_Q W_Q^T for W (naux, nao, nocc) FP64, in place and without a transposed copy of W.
+def _kernel_update(W: torch.Tensor, out: torch.Tensor) -> bool:
+    """True when the exchange kernel can take W (naux, nao, nocc) and out: FP64 on one GPU, out a row-major
+    (nao, nao) matrix.  Its pointers carry neither a type nor a device, so everything else stays with torch."""
+    return (W.is_cuda and out.device == W.device and W.dtype == torch.float64 and out.dtype == torch.float64
+            and tuple(out.shape) == (W.shape[1], W.shape[1]) and (out.stride(1) == 1 and out.stride(0) >= W.shape[1]
+                                                                  or out.shape[0] <= 1)
+            and not (W.is_neg() or out.is_neg()))
 
-    On the GPU the library's symmetric kernel (``dfb_dsyrk``: half the multiply-adds of a full product, k
-    split over the chip); its two triangles differ by the rounding of their span sums."""
+
+def exchange_update(W: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
+    """out += sum_Q W_Q W_Q^T for W (naux, nao, nocc), without a transposed copy of W in FP64 on the GPU.
+
+    There the library's symmetric kernel runs (``dfb_dsyrk``: half the multiply-adds of a full product, k
+    split over the chip); its two triangles differ by the rounding of their span sums.  Other types and
+    layouts take the product of a transposed copy, with torch's type promotion."""
     naux, nao, nocc = W.shape
-    if not W.is_cuda:
+    if not _kernel_update(W, out):
         W2 = W.permute(1, 0, 2).reshape(nao, naux * nocc)
-        return out.addmm_(W2, W2.T)
+        out += W2 @ W2.T
+        return out
     W = W.contiguous()
-    rc = _lib.lib().dfb_dsyrk(nao, naux, nocc, _lib.ptr(W), nao * nocc, nocc, _lib.ptr(out), out.stride(0),
+    rc = _lib.lib().dfb_dsyrk(nao, naux, nocc, _lib.ptr(W), nao * nocc, nocc, _lib.ptr(out), max(out.stride(0), nao),
                               int(torch.cuda.current_stream(W.device).cuda_stream))
     _lib.check(rc, "dfb_dsyrk")
     return out
