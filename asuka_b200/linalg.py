@@ -14,6 +14,7 @@ naux^2 * ncol multiply-adds as the TRSM.
 from __future__ import annotations
 
 import torch
+from torch.utils._device import DeviceContext
 
 from . import _lib
 
@@ -26,7 +27,7 @@ def diag_block_inverses(L: torch.Tensor, nb: int = NB) -> list[torch.Tensor]:
     the identity per block otherwise."""
     n = L.shape[0]
     starts = range(0, n, nb)
-    if not (L.is_cuda and L.dtype == torch.float64 and nb % 32 == 0 and 32 <= nb <= 256):
+    if not (L.is_cuda and L.dtype == torch.float64 and nb % 32 == 0 and 32 <= nb <= 256) or _observed(L):
         out = []
         for r0 in starts:
             r1 = min(n, r0 + nb)
@@ -85,6 +86,24 @@ def solve_lower_right_T(L: torch.Tensor, X: torch.Tensor, inv: list[torch.Tensor
     return B
 
 
+def _observed(*tensors: torch.Tensor) -> bool:
+    """True when something follows the operations on these tensors that a kernel on raw pointers would pass by:
+    autograd, forward-mode or function transforms, a tensor subclass, a mode or a tracer."""
+    if torch.is_grad_enabled() and any(t.requires_grad for t in tensors):
+        return True
+    if any(type(t) not in (torch.Tensor, torch.nn.Parameter) for t in tensors):
+        return True
+    if torch._C._functorch.maybe_current_level() is not None or torch.compiler.is_compiling() or torch.jit.is_tracing():
+        return True
+    if torch._C._len_torch_dispatch_stack():
+        return True
+    if torch._C._len_torch_function_stack():  # a default device is a mode too, which only creates tensors
+        if any(not isinstance(m, DeviceContext) for m in torch.overrides._get_current_function_mode_stack()):
+            return True
+    fw = torch.autograd.forward_ad
+    return fw._current_level >= 0 and any(fw.unpack_dual(t).tangent is not None for t in tensors)
+
+
 def _kernel_update(W: torch.Tensor, out: torch.Tensor) -> bool:
     """True when the exchange kernel can take W (naux, nao, nocc) and out: FP64 on one GPU, out a row-major
     (nao, nao) matrix.  Its pointers carry neither a type nor a device, so everything else stays with torch."""
@@ -99,9 +118,10 @@ def exchange_update(W: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
 
     There the library's symmetric kernel runs (``dfb_dsyrk``: half the multiply-adds of a full product, k
     split over the chip); its two triangles differ by the rounding of their span sums.  Other types and
-    layouts take the product of a transposed copy, with torch's type promotion."""
+    layouts, and tensors that autograd or a transform follows, take the product of a transposed copy, with
+    torch's type promotion."""
     naux, nao, nocc = W.shape
-    if not _kernel_update(W, out):
+    if not _kernel_update(W, out) or _observed(W, out):
         W2 = W.permute(1, 0, 2).reshape(nao, naux * nocc)
         out += W2 @ W2.T
         return out
@@ -109,4 +129,6 @@ def exchange_update(W: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
     rc = _lib.lib().dfb_dsyrk(nao, naux, nocc, _lib.ptr(W), nao * nocc, nocc, _lib.ptr(out), max(out.stride(0), nao),
                               int(torch.cuda.current_stream(W.device).cuda_stream))
     _lib.check(rc, "dfb_dsyrk")
+    if not out.is_inference():
+        torch.autograd.graph.increment_version(out)  # written behind autograd's back
     return out

@@ -84,3 +84,88 @@ def test_the_kernel_takes_fp64_of_one_gpu_only():
     for bad in (t((6, 6), dtype=torch.float32), t((6, 6), stride=(1, 6)), t((6, 6), stride=(0, 1)), t((5, 6)),
                 t((6, 6), neg=True)):
         assert not _kernel_update(W, bad)
+
+
+@pytest.mark.parametrize("device", DEVICES)
+def test_k_is_differentiable(device):
+    """K carries its graph, as J does: d/dCw and d/dBQ of <T, K> against the closed forms 2 sum_Q B_Q Ts B_Q Cw
+    and 2 Ts B_Q Cw Cw^T (Ts = (T + T^T) / 2, B_Q taken as independent elements: right factor Cw Cw^T)."""
+    from asuka_b200.jk import df_JK_from_BQ, df_K_from_BQ_Cw
+
+    B, Cw = _inputs(device)
+    T = torch.arange(NAO * NAO, dtype=torch.float64, device=device).reshape(NAO, NAO).cos()
+    Ts = 0.5 * (T + T.T)
+    C = Cw.clone().requires_grad_(True)
+    (gC,) = torch.autograd.grad((df_K_from_BQ_Cw(B, C) * T).sum(), C)
+    ref = 2.0 * torch.einsum("qmn,mk,qkl,li->ni", B, Ts, B, Cw)
+    assert float((gC - ref).abs().max()) <= 1e-12 * float(ref.abs().max())
+    Bg = B.clone().requires_grad_(True)
+    (gB,) = torch.autograd.grad((df_K_from_BQ_Cw(Bg, Cw) * T).sum(), Bg)
+    ref = 2.0 * torch.einsum("mk,qkl,li,ni->qmn", Ts, B, Cw, Cw)
+    assert float((gB - ref).abs().max()) <= 1e-12 * float(ref.abs().max())
+    J, K = df_JK_from_BQ(B, C, C @ C.T)
+    assert J.requires_grad and K.requires_grad
+    with torch.no_grad():
+        assert not df_K_from_BQ_Cw(B, C).requires_grad
+
+
+@pytest.mark.parametrize("device", DEVICES)
+def test_forward_mode_and_hooks(device):
+    """The tangent of K along a direction of Cw, by dual numbers and by ``torch.func.jvp``, and saved-tensor
+    hooks on the way."""
+    import torch.autograd.forward_ad as fwd
+
+    from asuka_b200.jk import df_K_from_BQ_Cw
+
+    B, Cw = _inputs(device)
+    V = Cw.sin()
+    U, dU = torch.matmul(B, Cw), torch.matmul(B, V)
+    ref = torch.einsum("qmi,qni->mn", U, dU)
+    ref = ref + ref.T
+    with fwd.dual_level():
+        K = df_K_from_BQ_Cw(B, fwd.make_dual(Cw, V))
+        dK = fwd.unpack_dual(K).tangent
+    assert float((dK - ref).abs().max()) <= 1e-12 * float(ref.abs().max())
+    _K, dK = torch.func.jvp(lambda c: df_K_from_BQ_Cw(B, c), (Cw,), (V,))
+    assert float((dK - ref).abs().max()) <= 1e-12 * float(ref.abs().max())
+    packed = []
+    C = Cw.clone().requires_grad_(True)
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: packed.append(t.shape) or t, lambda t: t):
+        df_K_from_BQ_Cw(B, C)
+    assert packed
+
+
+@pytest.mark.gpu
+def test_written_accumulator_is_noted():
+    """An accumulator that autograd saved before the kernel wrote to it is refused in backward, as for torch's
+    in-place sums; a default device does not take the kernel away."""
+    from asuka_b200 import _lib
+    from asuka_b200.linalg import exchange_update
+
+    B, Cw = _inputs("cuda")
+    W = torch.matmul(B, Cw)
+    out = torch.zeros((NAO, NAO), dtype=torch.float64, device="cuda")
+    x = torch.ones((NAO, NAO), dtype=torch.float64, device="cuda", requires_grad=True)
+    y = (x * out).sum()
+    L = _lib.lib()
+    with torch.device("cuda"):
+        n = L.dfb_launch_count()
+        exchange_update(W, out)
+        assert L.dfb_launch_count() > n
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        y.backward()
+
+
+@pytest.mark.parametrize("device", DEVICES)
+def test_block_inverses_are_differentiable(device):
+    """d/dL of <T, inverse of a diagonal block> = -(inv^T T inv^T) on the block."""
+    from asuka_b200.linalg import diag_block_inverses
+
+    n = 40
+    A = torch.randn((n, n + 4), generator=torch.Generator().manual_seed(2), dtype=torch.float64)
+    L = torch.linalg.cholesky(A @ A.T).to(device).requires_grad_(True)
+    T = torch.arange(32.0 * 32, dtype=torch.float64, device=device).reshape(32, 32).cos()
+    inv = diag_block_inverses(L, 32)[0]
+    (g,) = torch.autograd.grad((inv * T).sum(), L)
+    ref = -(inv.detach().T @ T @ inv.detach().T).tril()
+    assert float((g[:32, :32].tril() - ref).abs().max()) <= 1e-10 * float(ref.abs().max())
