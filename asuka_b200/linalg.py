@@ -34,10 +34,9 @@ def diag_block_inverses(L: torch.Tensor, nb: int = NB) -> list[torch.Tensor]:
             eye = torch.eye(r1 - r0, dtype=L.dtype, device=L.device)
             out.append(torch.linalg.solve_triangular(L[r0:r1, r0:r1], eye, upper=False))
         return out
-    Lr = L if L.stride(1) == 1 else L.contiguous()  # cuSOLVER returns its factor column-major
+    Lr = L if L.stride(1) == 1 and L.stride(0) >= n else L.contiguous()  # cuSOLVER returns its factor column-major
     inv = torch.empty((len(starts), nb, nb), dtype=L.dtype, device=L.device)
-    rc = _lib.lib().dfb_tri_inv(n, nb, _lib.ptr(Lr), Lr.stride(0), _lib.ptr(inv),
-                                int(torch.cuda.current_stream(L.device).cuda_stream))
+    rc = _launch(L.device, _lib.lib().dfb_tri_inv, n, nb, _lib.ptr(Lr), max(Lr.stride(0), n), _lib.ptr(inv))
     _lib.check(rc, "dfb_tri_inv")
     return [inv[i, : min(n, r0 + nb) - r0, : min(n, r0 + nb) - r0] for i, r0 in enumerate(starts)]
 
@@ -86,6 +85,16 @@ def solve_lower_right_T(L: torch.Tensor, X: torch.Tensor, inv: list[torch.Tensor
     return B
 
 
+def _launch(device: torch.device, fn, *args) -> int:
+    """fn(*args, the device's current stream) with that device current: a kernel is launched on the current
+    device, and its stream has to belong to it."""
+    stream = int(torch.cuda.current_stream(device).cuda_stream)
+    if device.index in (None, torch.cuda.current_device()):
+        return fn(*args, stream)
+    with torch.cuda.device(device):
+        return fn(*args, stream)
+
+
 def _observed(*tensors: torch.Tensor) -> bool:
     """True when something follows the operations on these tensors that a kernel on raw pointers would pass by:
     autograd, forward-mode or function transforms, a tensor subclass, a mode or a tracer."""
@@ -126,8 +135,8 @@ def exchange_update(W: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
         out += W2 @ W2.T
         return out
     W = W.contiguous()
-    rc = _lib.lib().dfb_dsyrk(nao, naux, nocc, _lib.ptr(W), nao * nocc, nocc, _lib.ptr(out), max(out.stride(0), nao),
-                              int(torch.cuda.current_stream(W.device).cuda_stream))
+    rc = _launch(W.device, _lib.lib().dfb_dsyrk, nao, naux, nocc, _lib.ptr(W), nao * nocc, nocc, _lib.ptr(out),
+                 max(out.stride(0), nao))
     _lib.check(rc, "dfb_dsyrk")
     if not out.is_inference():
         torch.autograd.graph.increment_version(out)  # written behind autograd's back

@@ -169,3 +169,41 @@ def test_block_inverses_are_differentiable(device):
     (g,) = torch.autograd.grad((inv * T).sum(), L)
     ref = -(inv.detach().T @ T @ inv.detach().T).tril()
     assert float((g[:32, :32].tril() - ref).abs().max()) <= 1e-10 * float(ref.abs().max())
+
+
+def test_launches_enter_the_tensors_device(monkeypatch):
+    """The launch helper with recorded torch.cuda calls: the tensors' device is made current around the call
+    when it is not, and the stream is that device's."""
+    from contextlib import contextmanager
+    from types import SimpleNamespace as NS
+
+    from asuka_b200 import linalg
+
+    state = {"current": 0}
+
+    @contextmanager
+    def device(d):
+        was, state["current"] = state["current"], d.index
+        yield
+        state["current"] = was
+
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: state["current"])
+    monkeypatch.setattr(torch.cuda, "device", device)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda d: NS(cuda_stream=100 + d.index))
+    for idx in (0, 1):
+        assert linalg._launch(torch.device("cuda", idx), lambda x, st: (x, st, state["current"]), 7) == (7, 100 + idx, idx)
+        assert state["current"] == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs two GPUs")
+def test_tensors_of_another_device():
+    from asuka_b200.jk import df_K_from_BQ_Cw
+    from asuka_b200.linalg import diag_block_inverses
+
+    B, Cw = _inputs("cuda:1")
+    with torch.cuda.device(0):
+        K = df_K_from_BQ_Cw(B, Cw)
+        (inv,) = diag_block_inverses(torch.eye(32, dtype=torch.float64, device="cuda:1"), 32)
+    assert float((K - _k(B, Cw)).abs().max()) <= 1e-13 * float(K.abs().max())
+    assert float((inv - torch.eye(32, dtype=torch.float64, device="cuda:1")).abs().max()) == 0.0
