@@ -207,3 +207,43 @@ def test_tensors_of_another_device():
         (inv,) = diag_block_inverses(torch.eye(32, dtype=torch.float64, device="cuda:1"), 32)
     assert float((K - _k(B, Cw)).abs().max()) <= 1e-13 * float(K.abs().max())
     assert float((inv - torch.eye(32, dtype=torch.float64, device="cuda:1")).abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("device", DEVICES)
+@pytest.mark.parametrize("precision", ["fp64", pytest.param("mixed", marks=pytest.mark.gpu)])
+def test_blocks_within_the_memory_there_is(monkeypatch, device, precision):
+    """Larger blocks than q_block only up to a quarter of B, never for factors whose blocks are copied, and none
+    where they cannot be allocated: a build that q_block rows fit runs through."""
+    from asuka_b200 import jk
+
+    if precision == "mixed" and device == "cpu":
+        pytest.skip("tensor-core products take CUDA tensors")
+    B, Cw = _inputs(device)
+    ref = _k(B, Cw)
+    tol = 1e-13 if precision == "fp64" else 1e-5
+    owner = torch if precision == "fp64" else jk._tc
+    product, rows = owner.matmul, []
+
+    def limited(limit):
+        def matmul(A, *a, **k):
+            if A.shape[0] > limit * NAO:
+                raise torch.OutOfMemoryError("no room")
+            rows.append(A.shape[0] // NAO)
+            return product(A, *a, **k)
+        return matmul
+
+    for factors, limit, most in ((B, NAUX, NAUX), (B, 7, 7), (B.permute(1, 2, 0).contiguous().permute(2, 0, 1), NAUX, 7)):
+        rows.clear()
+        with monkeypatch.context() as m:
+            m.setattr(owner, "matmul", limited(limit))
+            K = jk.df_K_from_BQ_Cw(factors, Cw, q_block=7, precision=precision)
+        assert max(rows) == most and sum(rows) == NAUX
+        assert float((K - ref).abs().max()) <= tol * float(ref.abs().max())
+    with monkeypatch.context() as m:
+        m.setattr(owner, "matmul", limited(6))
+        with pytest.raises(torch.OutOfMemoryError):
+            jk.df_K_from_BQ_Cw(B, Cw, q_block=7, precision=precision)
+    wide = torch.ones((NAO, 2 * NAO), dtype=torch.float64, device=device)  # U of all rows: twice B
+    assert jk._half_rows(B, wide.shape[1], 1) * NAO * wide.shape[1] <= B.numel() // 4
+    with pytest.raises(ValueError):
+        jk.df_K_from_BQ_Cw(B, Cw, q_block=0, precision=precision)
