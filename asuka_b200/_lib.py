@@ -99,6 +99,9 @@ _SIGS = {
                                       ctypes.c_long, ctypes.c_long, _d]),
     "dfb_dsyrk": (ctypes.c_int, [ctypes.c_int, ctypes.c_long, ctypes.c_long, _d, ctypes.c_long, ctypes.c_long, _d,
                                  ctypes.c_long, _d]),
+    "dfb_dsyrk_scratch": (ctypes.c_long, [ctypes.c_int, ctypes.c_long, ctypes.c_long]),
+    "dfb_dsyrk_ws": (ctypes.c_int, [ctypes.c_int, ctypes.c_long, ctypes.c_long, _d, ctypes.c_long, ctypes.c_long, _d,
+                                    ctypes.c_long, _d, ctypes.c_long, _d]),
     "dfb_tri_inv": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, _d, ctypes.c_long, _d, _d]),
     "dfb_launch_count": (ctypes.c_long, []),
     "dfb_rys_scratch_doubles": (ctypes.c_long, [ctypes.c_int] * 3 + [ctypes.c_long, ctypes.c_int]),

@@ -128,18 +128,26 @@ __global__ void __launch_bounds__(NT, 3) k_gamma_sym(long nP, int nao, int nocc,
 
 // Exchange update K += sum_k A(m, k) A(n, k) of the FP64 path, A(m, k) = W[kq * skq + m * sm + k1] with
 // k = kq * nk1 + k1 (W[Q, mu, i]: skq = nao nocc, sm = nocc, nk1 = nocc), so W is read in place.
-// FP64-FMA-bound.  Only the 64 x 64 tiles on and above the diagonal are formed (0.57 of a full product at
-// nao 416) and k is cut into spans over blockIdx.y, so that a few hundred columns still fill the chip;
-// the spans add into K atomically, off-diagonal tiles in both orders.  128 threads, 8 x 4 outputs each
-// (12 shared-memory reads per 32 multiply-adds), k chunks of 16 double-buffered through registers.
-// nao 416, k 72960: 1.03 ms (26 TFLOP/s); a transposed copy and the library's full product took 1.4 to 1.5 ms.
+// Only the 64 x 64 tiles on and above the diagonal are formed (0.57 of a full product at nao 416) and k is
+// cut into spans over blockIdx.y, so that a few hundred columns still fill the chip.  A launch takes one full
+// wave of spans of at most SFL terms (short chains of roundings: relative error 2.3e-16 at k 72960, 8.1e-16 with
+// spans of 3300); each block adds its sums to its own tile of `part`, and k_dsyrk_sum adds the spans in their
+// order, so K repeats itself bit for bit.  128 threads, 8 x 4 outputs each, k chunks of 16 double-buffered
+// through registers: 12 eight-byte shared-memory reads per 32 multiply-adds and the 128 registers that four
+// blocks per SM leave bound it, not the FP64 pipe.  nao 416, k 72960: 8.4 G multiply-adds with the padding and
+// the whole diagonal tiles in 0.98 ms, 17 of 34 TFLOP/s (spans over all k and atomic sums 1.04; a transposed
+// copy and the library's full product 1.4 to 1.5); nao 624, k 164160: 4.46 (4.71); nao 208, k 18240: 0.099 (0.116).
+// part = nullptr: the sums go to C by atomic additions (several spans: in any order).
 constexpr int ST = 64;        // tile edge
 constexpr int SKC = 16;       // k per chunk
 constexpr int SNT = 128;      // threads
+constexpr int SFL = 512;      // most terms of a span
+constexpr int SMIN = 128;     // least terms of a span, which ends in 64 x 64 sums (nao 58, k 2300: 512 50 us, 256 32, 128 24)
 constexpr int SP = ST + 1;    // row stride of a chunk: the transposing stores of a half warp hit 16 banks
 
-__global__ void __launch_bounds__(SNT, 4) k_dsyrk(int n, long K, long nk1, const double* __restrict__ W, long skq, long sm,
-                                               double* __restrict__ C, long ldc, long kspan, int T) {
+__global__ void __launch_bounds__(SNT, 4) k_dsyrk(int n, long k_lo, long k_hi, long nk1, const double* __restrict__ W,
+                                                  long skq, long sm, double* __restrict__ C, long ldc, long kspan, int T,
+                                                  double* __restrict__ part) {
     __shared__ double sA[2][SKC * SP], sB[2][SKC * SP];
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     int idx = blockIdx.x, mt = 0;
@@ -149,7 +157,7 @@ __global__ void __launch_bounds__(SNT, 4) k_dsyrk(int n, long K, long nk1, const
     }
     const int nt = mt + idx, m0 = mt * ST, n0 = nt * ST;
     const bool diag = mt == nt;
-    const long kbeg = (long)blockIdx.y * kspan, kend = kbeg + kspan < K ? kbeg + kspan : K;
+    const long kbeg = k_lo + (long)blockIdx.y * kspan, kend = kbeg + kspan < k_hi ? kbeg + kspan : k_hi;
     const int lk = tid & (SKC - 1), lr = tid >> 4;  // this thread loads column lk of rows lr + 8 i
     double va[8], vb[8];
     auto load = [&](long k0) {
@@ -201,6 +209,17 @@ __global__ void __launch_bounds__(SNT, 4) k_dsyrk(int n, long K, long nk1, const
         __syncthreads();
         buf ^= 1;
     }
+    if (part) {
+        double* own = part + ((long)blockIdx.y * gridDim.x + blockIdx.x) * (ST * ST) + tid;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                double* q = own + (i * 4 + j) * SNT;
+                *q = k_lo == 0 ? acc[i][j] : *q + acc[i][j];
+            }
+        return;
+    }
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         const int m = m0 + 8 * ty + i;
@@ -213,6 +232,57 @@ __global__ void __launch_bounds__(SNT, 4) k_dsyrk(int n, long K, long nk1, const
             if (c != m) atomicAdd(C + (long)c * ldc + m, acc[i][j]);
         }
     }
+}
+
+// C += the spans of one tile, in their order: thread = element, both orders of an off-diagonal pair.
+__global__ void __launch_bounds__(256) k_dsyrk_sum(int n, int ns, const double* __restrict__ part, double* __restrict__ C,
+                                                   long ldc, int T) {
+    int idx = blockIdx.x, mt = 0;
+    while (idx >= T - mt) {
+        idx -= T - mt;
+        ++mt;
+    }
+    const int e = blockIdx.y * 256 + threadIdx.x, r = e / SNT, tid = e % SNT;
+    const int m = mt * ST + 8 * (tid >> 4) + r / 4, c = (mt + idx) * ST + (tid & 15) + 16 * (r % 4);
+    if (m >= n || c >= n || (idx == 0 && c < m)) return;
+    const double* p = part + (long)blockIdx.x * (ST * ST) + e;
+    double v = 0.0;
+#pragma unroll 8
+    for (int s = 0; s < ns; ++s) v += p[(long)s * gridDim.x * (ST * ST)];
+    C[(long)m * ldc + c] += v;
+    if (c != m) C[(long)c * ldc + m] += v;
+}
+
+// The launches of an exchange update of n rows: `nslab` slabs of k, each `ns` spans.
+struct SyrkPlan {
+    int T;
+    long ntiles, ns, span, nslab;
+};
+static SyrkPlan syrk_plan(int n, long K, bool one_launch) {
+    SyrkPlan p;
+    p.T = (n + ST - 1) / ST;
+    p.ntiles = (long)p.T * (p.T + 1) / 2;
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const long slots = 4L * sms;  // blocks resident at a time
+    // full waves: the span count rounded down, over as few waves (up to three) as leave less than a tenth idle
+    p.ns = 1;
+    double best = 0.0;
+    for (int w = 1; w <= 3 && best < 0.9; ++w) {
+        const long ns = w * slots / p.ntiles;
+        const double use = (double)ns * p.ntiles / ((double)w * slots);
+        if (ns >= 1 && use > best + 0.02) {
+            best = use;
+            p.ns = ns;
+        }
+    }
+    const long most = (K + SMIN - 1) / SMIN;
+    if (p.ns > most) p.ns = most;
+    p.nslab = one_launch ? 1 : (K + p.ns * SFL - 1) / (p.ns * SFL);
+    p.span = (K + p.nslab * p.ns - 1) / (p.nslab * p.ns);
+    p.span = (p.span + SKC - 1) / SKC * SKC;
+    if (p.nslab == 1) p.ns = (K + p.span - 1) / p.span;
+    return p;
 }
 
 // Inverses of the nb x nb diagonal blocks of a lower-triangular L by forward substitution.  A CTA takes 32
@@ -323,29 +393,50 @@ extern "C" int dfb_gamma_sym(long nP, int nao, int nocc, const double* U, long s
     return DFB_OK;
 }
 
-extern "C" int dfb_dsyrk(int n, long nkq, long nk1, const double* W, long skq, long sm, double* C, long ldc, void* stream) {
+extern "C" long dfb_dsyrk_scratch(int n, long nkq, long nk1) {
+    if (n <= 0 || nkq <= 0 || nk1 <= 0) return 0;
+    const dense::SyrkPlan p = dense::syrk_plan(n, nkq * nk1, false);
+    return p.ns * p.nslab > 1 ? p.ns * p.ntiles * dense::ST * dense::ST : 0;
+}
+
+extern "C" int dfb_dsyrk_ws(int n, long nkq, long nk1, const double* W, long skq, long sm, double* C, long ldc,
+                            double* ws, long ws_doubles, void* stream) {
     clear_error();
     if (n < 0 || nkq < 0 || nk1 < 0 || ldc < n)
         return set_error(DFB_ERR_INVALID, "invalid sizes to dfb_dsyrk (n %d, k %ld x %ld)", n, nkq, nk1);
     const long K = nkq * nk1;
     if (n == 0 || K == 0) return DFB_OK;
     if (!W || !C) return set_error(DFB_ERR_INVALID, "invalid pointers to dfb_dsyrk");
-    const int T = (n + dense::ST - 1) / dense::ST;
-    const long ntiles = (long)T * (T + 1) / 2;
-    if (ntiles > 0x7fffffffL) return set_error(DFB_ERR_UNSUPPORTED, "n %d too large", n);
-    // spans: about four resident blocks per SM, each at least 512 long (a span ends in 64 x 64 atomic additions)
-    long ns = (4 * 148 + ntiles - 1) / ntiles;
-    if (ns > (K + 511) / 512) ns = (K + 511) / 512;
-    if (ns < 1) ns = 1;
-    long span = (K + ns - 1) / ns;
-    span = (span + dense::SKC - 1) / dense::SKC * dense::SKC;
-    ns = (K + span - 1) / span;
-    dense::k_dsyrk<<<dim3((unsigned)ntiles, (unsigned)ns), dense::SNT, 0, (cudaStream_t)stream>>>(n, K, nk1, W, skq, sm, C,
-                                                                                                  ldc, span, T);
-    count_launches(1);
-    cudaError_t e = cudaGetLastError();
+    const dense::SyrkPlan p = dense::syrk_plan(n, K, !ws);
+    if (p.ntiles > 0x7fffffffL) return set_error(DFB_ERR_UNSUPPORTED, "n %d too large", n);
+    if (p.ns * p.nslab == 1) ws = nullptr;  // one span: no sums to add
+    if (ws && ws_doubles < p.ns * p.ntiles * dense::ST * dense::ST)
+        return set_error(DFB_ERR_INVALID, "dfb_dsyrk needs %ld scratch doubles, %ld given",
+                         p.ns * p.ntiles * dense::ST * dense::ST, ws_doubles);
+    cudaStream_t st = (cudaStream_t)stream;
+    cudaError_t e = cudaSuccess;
+    const long slab = p.ns * p.span;
+    for (long k0 = 0; k0 < K && e == cudaSuccess; k0 += slab) {
+        // the last slab may leave spans without terms: they keep what their tiles of ws hold
+        const long k1 = k0 + slab < K ? k0 + slab : K, ny = (k1 - k0 + p.span - 1) / p.span;
+        dense::k_dsyrk<<<dim3((unsigned)p.ntiles, (unsigned)ny), dense::SNT, 0, st>>>(n, k0, k1, nk1, W, skq, sm, C, ldc,
+                                                                                      p.span, p.T, ws);
+        count_launches(1);
+        e = cudaGetLastError();
+    }
     if (e != cudaSuccess) return set_cuda_error("k_dsyrk launch", e);
+    if (ws) {
+        dense::k_dsyrk_sum<<<dim3((unsigned)p.ntiles, dense::ST * dense::ST / 256), 256, 0, st>>>(n, (int)p.ns, ws, C, ldc,
+                                                                                                 p.T);
+        count_launches(1);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return set_cuda_error("k_dsyrk_sum launch", e);
+    }
     return DFB_OK;
+}
+
+extern "C" int dfb_dsyrk(int n, long nkq, long nk1, const double* W, long skq, long sm, double* C, long ldc, void* stream) {
+    return dfb_dsyrk_ws(n, nkq, nk1, W, skq, sm, C, ldc, nullptr, 0, stream);
 }
 
 extern "C" int dfb_tri_inv(int n, int nb, const double* L, long ldl, double* out, void* stream) {

@@ -13,12 +13,16 @@ naux^2 * ncol multiply-adds as the TRSM.
 
 from __future__ import annotations
 
+import functools
+
 import torch
+import torch.autograd.forward_ad as _fwd
 from torch.utils._device import DeviceContext
 
 from . import _lib
 
 NB = 256  # rows per diagonal block
+_PLAIN = (torch.Tensor, torch.nn.Parameter)
 
 
 def diag_block_inverses(L: torch.Tensor, nb: int = NB) -> list[torch.Tensor]:
@@ -98,19 +102,18 @@ def _launch(device: torch.device, fn, *args) -> int:
 def _observed(*tensors: torch.Tensor) -> bool:
     """True when something follows the operations on these tensors that a kernel on raw pointers would pass by:
     autograd, forward-mode or function transforms, a tensor subclass, a mode or a tracer."""
-    if torch.is_grad_enabled() and any(t.requires_grad for t in tensors):
+    grad = torch.is_grad_enabled()
+    for t in tensors:
+        if type(t) not in _PLAIN or (grad and t.requires_grad):
+            return True
+    c = torch._C
+    if (c._functorch.maybe_current_level() is not None or c._len_torch_dispatch_stack() or torch.compiler.is_compiling()
+            or c._get_tracing_state() is not None):
         return True
-    if any(type(t) not in (torch.Tensor, torch.nn.Parameter) for t in tensors):
-        return True
-    if torch._C._functorch.maybe_current_level() is not None or torch.compiler.is_compiling() or torch.jit.is_tracing():
-        return True
-    if torch._C._len_torch_dispatch_stack():
-        return True
-    if torch._C._len_torch_function_stack():  # a default device is a mode too, which only creates tensors
+    if c._len_torch_function_stack():  # a default device is a mode too, which only creates tensors
         if any(not isinstance(m, DeviceContext) for m in torch.overrides._get_current_function_mode_stack()):
             return True
-    fw = torch.autograd.forward_ad
-    return fw._current_level >= 0 and any(fw.unpack_dual(t).tangent is not None for t in tensors)
+    return _fwd._current_level >= 0 and any(_fwd.unpack_dual(t).tangent is not None for t in tensors)
 
 
 def _kernel_update(W: torch.Tensor, out: torch.Tensor) -> bool:
@@ -122,11 +125,17 @@ def _kernel_update(W: torch.Tensor, out: torch.Tensor) -> bool:
             and not (W.is_neg() or out.is_neg()))
 
 
+@functools.lru_cache(maxsize=256)
+def _syrk_scratch(nao: int, naux: int, nocc: int, device: int) -> int:
+    with torch.cuda.device(device):
+        return int(_lib.lib().dfb_dsyrk_scratch(nao, naux, nocc))
+
+
 def exchange_update(W: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
     """out += sum_Q W_Q W_Q^T for W (naux, nao, nocc), without a transposed copy of W in FP64 on the GPU.
 
     There the library's symmetric kernel runs (``dfb_dsyrk``: half the multiply-adds of a full product, k
-    split over the chip); its two triangles differ by the rounding of their span sums.  Other types and
+    split over the chip and its spans added in a fixed order: equal calls give equal bits).  Other types and
     layouts, and tensors that autograd or a transform follows, take the product of a transposed copy, with
     torch's type promotion."""
     naux, nao, nocc = W.shape
@@ -135,8 +144,11 @@ def exchange_update(W: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
         out += W2 @ W2.T
         return out
     W = W.contiguous()
-    rc = _launch(W.device, _lib.lib().dfb_dsyrk, nao, naux, nocc, _lib.ptr(W), nao * nocc, nocc, _lib.ptr(out),
-                 max(out.stride(0), nao))
+    device = W.device
+    need = _syrk_scratch(nao, naux, nocc, device.index)
+    ws = torch.empty(need, dtype=torch.float64, device=device) if need else None  # freed in stream order
+    rc = _launch(device, _lib.lib().dfb_dsyrk_ws, nao, naux, nocc, W.data_ptr(), nao * nocc, nocc, out.data_ptr(),
+                 max(out.stride(0), nao), _lib.ptr(ws), need)
     _lib.check(rc, "dfb_dsyrk")
     if not out.is_inference():
         torch.autograd.graph.increment_version(out)  # written behind autograd's back

@@ -284,9 +284,14 @@ int dfb_prim_integrals(const dfb_bra_t *bra, const dfb_groups_t *groups, const d
 
 /*
  * FP64 exchange update C[m*ldc + n] += sum_k A(m, k) A(n, k), A(m, k) = W[(k / nk1)*skq + m*sm + k % nk1]
- * with k < nkq*nk1 (W[Q, mu, i]: skq = nao*nocc, sm = nocc, nk1 = nocc).  Adds with FP64 atomics, both
- * orders.  Replaces the cuBLAS products of hf_df_jk_cuda_ext.cpp:231-598 in FP64.
+ * with k < nkq*nk1 (W[Q, mu, i]: skq = nao*nocc, sm = nocc, nk1 = nocc), both orders.  With a workspace of
+ * dfb_dsyrk_scratch doubles (0: none is used) the k spans are added in a fixed order, so equal calls give equal
+ * bits on one type of GPU; without one (dfb_dsyrk) by FP64 atomics.  Replaces the cuBLAS products of
+ * hf_df_jk_cuda_ext.cpp:231-598 in FP64.
  */
+long dfb_dsyrk_scratch(int n, long nkq, long nk1);
+int dfb_dsyrk_ws(int n, long nkq, long nk1, const double *W, long skq, long sm, double *C, long ldc, double *ws,
+                 long ws_doubles, void *stream);
 int dfb_dsyrk(int n, long nkq, long nk1, const double *W, long skq, long sm, double *C, long ldc, void *stream);
 
 /*

@@ -247,3 +247,66 @@ def test_blocks_within_the_memory_there_is(monkeypatch, device, precision):
     assert jk._half_rows(B, wide.shape[1], 1) * NAO * wide.shape[1] <= B.numel() // 4
     with pytest.raises(ValueError):
         jk.df_K_from_BQ_Cw(B, Cw, q_block=0, precision=precision)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("naux,nao,nocc", [(3, 5, 1), (40, 64, 13), (900, 65, 7), (700, 70, 40), (333, 300, 11), (60, 1100, 3)])
+def test_exchange_sum_repeats_and_stays_close(naux, nao, nocc):
+    """Equal calls give equal bits and a symmetric sum, beside each other on two streams too.  Error: chains of
+    at most 512 terms, then the sums of a span and of the spans; 512 + K/512 roundings of random sign stay below
+    4 sqrt(512 + K/512) ulp of the magnitudes summed."""
+    from asuka_b200.linalg import exchange_update
+
+    g = torch.Generator(device="cuda")
+    g.manual_seed(nao)
+    W = torch.randn((naux, nao, nocc), generator=g, dtype=torch.float64, device="cuda")
+
+    def run():
+        return exchange_update(W, torch.zeros((nao, nao), dtype=torch.float64, device="cuda"))
+
+    K = run()
+    assert torch.equal(K, K.T)
+    for _ in range(3):
+        assert torch.equal(run(), K)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        K1 = run()
+    K2 = run()
+    torch.cuda.synchronize()
+    assert torch.equal(K1, K) and torch.equal(K2, K)
+    rows = slice(0, min(nao, 96))
+    A = (W.permute(1, 0, 2).reshape(nao, -1).cpu())[rows]
+    ref = torch.zeros((A.shape[0], A.shape[0]), dtype=torch.float64)
+    comp = torch.zeros_like(ref)
+    for k0 in range(0, A.shape[1], 8):  # compensated sums of short products
+        p = A[:, k0:k0 + 8]
+        hi = p.float().double()
+        lo = p - hi
+        for t in (hi @ hi.T, hi @ lo.T, lo @ hi.T, lo @ lo.T):
+            y = t - comp
+            s = ref + y
+            comp = (s - ref) - y
+            ref = s
+    k = naux * nocc
+    mag = A.abs() @ A.abs().T
+    assert bool(((K.cpu()[rows, rows] - ref).abs() <= 4 * (512 + k / 512) ** 0.5 * 1.2e-16 * mag).all())
+
+
+@pytest.mark.gpu
+def test_exchange_workspace_is_checked():
+    from asuka_b200 import _lib
+
+    L = _lib.lib()
+    need = L.dfb_dsyrk_scratch(70, 700, 40)
+    assert need > 0 and L.dfb_dsyrk_scratch(5, 3, 1) == 0 and L.dfb_dsyrk_scratch(0, 3, 1) == 0
+    W = torch.ones((700, 70, 40), dtype=torch.float64, device="cuda")
+    C = torch.zeros((70, 70), dtype=torch.float64, device="cuda")
+    ws = torch.empty(need, dtype=torch.float64, device="cuda")
+    st = int(torch.cuda.current_stream().cuda_stream)
+    args = (70, 700, 40, W.data_ptr(), 2800, 40, C.data_ptr(), 70)
+    assert L.dfb_dsyrk_ws(*args, ws.data_ptr(), need - 1, st) == -1
+    assert L.dfb_dsyrk_ws(*args, ws.data_ptr(), need, st) == 0
+    assert L.dfb_dsyrk(*args, st) == 0  # without a workspace: atomics
+    torch.cuda.synchronize()
+    assert float((C - 2 * 28000.0).abs().max()) == 0.0
