@@ -133,8 +133,9 @@ __global__ void __launch_bounds__(NT, 3) k_gamma_sym(long nP, int nao, int nocc,
 // wave of spans of at most SFL terms (short chains of roundings: relative error 2.3e-16 at k 72960, 8.1e-16 with
 // spans of 3300); each block adds its sums to its own tile of `part`, and k_dsyrk_sum adds the spans in their
 // order, so K repeats itself bit for bit.  128 threads, 8 x 4 outputs each, k chunks of 16 double-buffered
-// through registers: 12 eight-byte shared-memory reads per 32 multiply-adds and the 128 registers that four
-// blocks per SM leave bound it, not the FP64 pipe.  nao 416, k 72960: 8.4 G multiply-adds with the padding and
+// through registers, 12 eight-byte shared-memory reads per 32 multiply-adds.  Neither unit is full: FP64 pipe
+// 52 %, shared-memory wavefronts 54 %, 0.49 instructions per cycle and scheduler from 12 warps per SM (128
+// registers leave four blocks).  nao 416, k 72960: 8.4 G multiply-adds with the padding and
 // the whole diagonal tiles in 0.98 ms, 17 of 34 TFLOP/s (spans over all k and atomic sums 1.04; a transposed
 // copy and the library's full product 1.4 to 1.5); nao 624, k 164160: 4.46 (4.71); nao 208, k 18240: 0.099 (0.116).
 // part = nullptr: the sums go to C by atomic additions (several spans: in any order).
