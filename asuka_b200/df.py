@@ -50,8 +50,8 @@ _SIDE_STREAMS: dict[int, list] = {}
 
 
 class ScratchHolder:
-    """Device scratch for the generic kernels, shared by engines that run one after another
-    on the same streams (a batch of molecules): one buffer, grown to the largest need."""
+    """Device scratch for the generic shell-by-shell kernels, shared by engines that run one after
+    another on the same streams (a batch of molecules): one buffer, grown to the largest need."""
 
     def __init__(self):
         self.t: torch.Tensor | None = None
@@ -254,7 +254,7 @@ class DFEngine:
         return main, side, arr
 
     def _join(self, fork) -> None:
-        main, side, arr = fork
+        main, side, arr = fork[:3]
         if side[0] is not main:
             _lib.check(_lib.lib().dfb_join(int(main.cuda_stream), arr, len(side)), "dfb_join")
 
@@ -649,29 +649,34 @@ class DFEngine:
 
     def _run_int(self, works, then=None):
         """Run the integral works over the side streams and join.  With a second set ``then`` the current
-        stream waits for the first set only; the fork is returned for ``_join``."""
+        stream waits for the first set only; the fork is returned for ``_join`` and holds the scratch until then.
+
+        The rows of primitive integrals belong to the call: they come from the allocator in the order of the
+        current stream (of the graph, under capture) and go back to it after the join, so calls from several
+        streams or threads and captured calls never share them."""
         L = _lib.lib()
         n = max(NSTREAMS, 1)
         every = works + (then or [])
-        need = max(w[4] for w in every)
-        need = max((need + 31) // 32 * 32 * n, n * 32)
         if any(w[7] for w in every):
-            need = max(need, self._scratch_for(False, copies=n).numel())
-        buf = self._scratch.get(need, self.device)
-        per = buf.numel() // n // 32 * 32
-        self._slices_int = [buf[i * per:(i + 1) * per] for i in range(n)]
-        fork = self._fork()
-        _main, side, streams = fork
-        for batch in (works, then or []):
-            for bra, groups, arr, ncls, _per, out, (sP, sM, sN), rest in batch:
-                if ncls:
-                    rc = L.dfb_prim_integrals(ctypes.byref(bra), ctypes.byref(groups.c), arr, ncls, _lib.ptr(out), sP, sM,
-                                              sN, _lib.ptr(buf), buf.numel(), streams, len(side))
-                    _lib.check(rc, "dfb_prim_integrals")
-                for i, job in enumerate(rest):
-                    self._launch_int(*job)(int(side[i % n].cuda_stream))
-            if batch is works:
-                self._join(fork)
+            self._slices_int = self._scratch_slices(False)
+        per = (max(w[4] for w in every) + 31) // 32 * 32
+        rows = torch.empty(n * per, dtype=torch.float64, device=self.device)
+        fork = (*self._fork(), rows)
+        _main, side, streams, _rows = fork
+        try:
+            for batch in (works, then or []):
+                for bra, groups, arr, ncls, _per, out, (sP, sM, sN), rest in batch:
+                    if ncls:
+                        rc = L.dfb_prim_integrals(ctypes.byref(bra), ctypes.byref(groups.c), arr, ncls, _lib.ptr(out), sP,
+                                                  sM, sN, _lib.ptr(rows), rows.numel(), streams, len(side))
+                        _lib.check(rc, "dfb_prim_integrals")
+                    for i, job in enumerate(rest):
+                        self._launch_int(*job)(int(side[i % n].cuda_stream))
+                if batch is works:
+                    self._join(fork)
+        except BaseException:
+            self._join(fork)  # what was launched still writes to its rows
+            raise
         return fork
 
     def _run_deriv(self, works, grad) -> None:
@@ -708,9 +713,11 @@ class DFEngine:
         X = X if X is not None else torch.empty((naux, nao, nao), dtype=torch.float64, device=self.device)
         self._clear_dropped(X, (nao * nao, nao, 1), naux)
         fork = self._run_int([self._metric_work(V)], [self._int3c_work(X, (nao * nao, nao, 1), precision)])
-        V.copy_(0.5 * (V + V.T))
-        L, info = torch.linalg.cholesky_ex(V)
-        self._join(fork)
+        try:
+            V.copy_(0.5 * (V + V.T))
+            L, info = torch.linalg.cholesky_ex(V)
+        finally:
+            self._join(fork)
         if int(info.item()) != 0:
             raise RuntimeError(f"metric Cholesky failed (leading minor {int(info.item())} not positive definite)")
         return V, L, X

@@ -1,0 +1,98 @@
+"""Scratch of the integral calls: rows of primitive integrals belong to one call."""
+
+import ctypes
+
+import pytest
+
+torch = pytest.importorskip("torch")
+
+
+class _FakeLib:
+    """Records the scratch range of every integral call."""
+
+    def __init__(self):
+        self.ranges = []
+
+    def dfb_prim_integrals(self, _bra, _groups, _arr, _ncls, _out, _sp, _sm, _sn, ptr, doubles, _streams, _n):
+        self.ranges.append((ptr, ptr + 8 * doubles))
+        return 0
+
+
+def _overlap(a, b):
+    return a[0] < b[1] and b[0] < a[1]
+
+
+def test_calls_in_flight_have_their_own_rows(monkeypatch):
+    """Two calls of one engine before the first has ended (its fork is open), larger and smaller needs first."""
+    from types import SimpleNamespace as NS
+
+    from asuka_b200 import _lib, df
+
+    fake = _FakeLib()
+    monkeypatch.setattr(_lib, "lib", lambda: fake)
+    eng = df.DFEngine.__new__(df.DFEngine)
+    eng.device = torch.device("cpu")
+    eng._scratch = df.ScratchHolder()
+    st = NS(cuda_stream=0)
+    monkeypatch.setattr(df.DFEngine, "_fork", lambda self: (st, [st] * 8, (ctypes.c_void_p * 8)()))
+    monkeypatch.setattr(df.DFEngine, "_join", lambda self, fork: None)
+    out = torch.zeros(1)
+    groups = NS(c=_lib.Groups())
+    for first, second in ((1000, 40), (40, 1000), (64, 64)):
+        fake.ranges.clear()
+        held = [eng._run_int([(_lib.Bra(), groups, None, 1, need, out, (0, 0, 0), [])]) for need in (first, second)]
+        a, b = fake.ranges
+        assert a[1] - a[0] >= 64 * first and b[1] - b[0] >= 64 * second  # eight slices of 8-byte doubles
+        assert not _overlap(a, b)
+        assert len(held) == 2
+
+
+def _engine(n=2):
+    from asuka_b200 import basis as bm
+    from asuka_b200 import geometry as geo
+    from asuka_b200.df import DFEngine
+
+    mol = geo.water_cluster(n, 3, "ma-svp")
+    atoms = list(mol.atoms_bohr)
+    return DFEngine(bm.pack_basis(atoms, mol.basis, "ao"), bm.pack_basis(atoms, mol.basis, "aux"))
+
+
+@pytest.mark.gpu
+def test_calls_from_two_streams():
+    """Metric and 3c integrals of one engine issued from two streams, whose kernels run beside each other."""
+    eng = _engine()
+    V0, X0 = eng.metric(), eng.int3c("Qmn")
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    for _ in range(5):
+        torch.cuda.synchronize()
+        with torch.cuda.stream(a):
+            torch.cuda._sleep(200000)
+            V = eng.metric()
+        with torch.cuda.stream(b):
+            X = eng.int3c("Qmn")
+        with torch.cuda.stream(a):
+            V2 = eng.metric()
+        torch.cuda.synchronize()
+        assert torch.equal(V, V0) and torch.equal(V2, V0) and torch.equal(X, X0)
+
+
+@pytest.mark.gpu
+def test_captured_call_outlives_larger_ones():
+    """A captured metric replayed after a call with a larger need, with the freed memory written over."""
+    eng = _engine()
+    V0 = eng.metric()
+    eng2 = _engine()
+    eng2.metric()
+    torch.cuda.synchronize()
+    V = torch.empty_like(V0)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        eng2.metric(out=V)
+    eng2.int3c("Qmn")
+    junk = [torch.full((1 << 20,), float("nan"), dtype=torch.float64, device="cuda") for _ in range(8)]
+    for _ in range(2):
+        V.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(V, V0)
+    assert all(bool(torch.isnan(t).all()) for t in junk)  # the replay wrote to none of it
