@@ -139,21 +139,27 @@ static long prim_row(int la, int lb, int lc) {
 
 using namespace dfb;
 
+// Doubles of one row over a tile of 32 pairs; the most rows of one group.
+static long tile_row(const dfb_prim_class_t& c) { return prim_row(c.la, c.lb, c.lc) * 32; }
+static long group_rows(const dfb_prim_class_t& c) {
+    long most = 0;
+    for (int k = 0; k < c.ngroup; ++k) most = c.rows[k + 1] - c.rows[k] > most ? c.rows[k + 1] - c.rows[k] : most;
+    return most;
+}
+
+// A wave holds whole groups over a range of pair tiles: `target` doubles bound it unless one group over one
+// tile takes more.  The metric contracts pairs of groups: its waves hold all pairs, whose count grows with the
+// primitives of one l only.
 extern "C" long dfb_prim_scratch(const dfb_prim_class_t* cls, int ncls, long target) {
     long need = 1;
     for (int i = 0; i < ncls; ++i) {
         const dfb_prim_class_t& c = cls[i];
         if (c.ngroup <= 0 || c.npair <= 0) continue;
-        const long row = prim_row(c.la, c.lb, c.lc) * (((long)c.npair + 31) / 32) * 32;
-        long big = 0;
-        for (int k = 0; k < c.ngroup; ++k) {
-            const long n = c.rows[k + 1] - c.rows[k];
-            if (n > big) big = n;
-        }
-        long rows = target / row;
-        if (rows < big) rows = big;
-        if (rows > c.rows[c.ngroup]) rows = c.rows[c.ngroup];
-        if (rows * row > need) need = rows * row;
+        const long tiles = ((long)c.npair + 31) / 32, one = tile_row(c) * (c.bra_groups ? tiles : 1);
+        const long least = group_rows(c) * one, all = c.rows[c.ngroup] * tile_row(c) * tiles;
+        long n = least > target ? least : target;
+        if (n > all) n = all;
+        if (n > need) need = n;
     }
     return need;
 }
@@ -172,8 +178,6 @@ extern "C" int dfb_prim_integrals(const dfb_bra_t* bra, const dfb_groups_t* gr, 
         if (!dfb_grad_supported(c.la, c.lb, c.lc, bra->b_dummy))
             return set_error(DFB_ERR_UNSUPPORTED, "integral class (%d,%d,%d) is not supported", c.la, c.lb, c.lc);
         if (c.npair <= 0 || c.ngroup <= 0) continue;
-        if (c.npair > 65535L * GRAD_THREADS)
-            return set_error(DFB_ERR_UNSUPPORTED, "class (%d,%d,%d) has too many pairs", c.la, c.lb, c.lc);
         if (!c.pairs || !c.chunks || !c.groups || !c.rows || !c.first_chunk || c.max_shells < 1 || (bra->b_dummy && !c.bra_groups))
             return set_error(DFB_ERR_INVALID, "integral class without lists");
         cudaStream_t st = (cudaStream_t)streams[i % nstreams];
@@ -190,9 +194,6 @@ extern "C" int dfb_prim_integrals(const dfb_bra_t* bra, const dfb_groups_t* gr, 
         g.rec = bra->rec;
         g.cxyz = bra->cxyz;
         g.b_dummy = bra->b_dummy;
-        g.pairs = c.pairs;
-        g.npair = c.npair;
-        g.ntile = (c.npair + 31) / 32;
         g.gg = {gr->info, gr->coef, gr->shells, gr->pexp, gr->rexp, gr->cxyz, gr->aostart, gr->atom};
         g.W = W;
         g.lc = c.lc;
@@ -203,9 +204,6 @@ extern "C" int dfb_prim_integrals(const dfb_bra_t* bra, const dfb_groups_t* gr, 
         m.shB = bra->shB;
         m.cxyz = bra->cxyz;
         m.aostart = bra->aostart;
-        m.pairs = c.pairs;
-        m.npair = c.npair;
-        m.ntile = g.ntile;
         m.gg = g.gg;
         m.W = W;
         m.out = out;
@@ -213,32 +211,51 @@ extern "C" int dfb_prim_integrals(const dfb_bra_t* bra, const dfb_groups_t* gr, 
         m.sM = sM;
         m.sN = sN;
         m.lc = c.lc;
-        const long row = prim_row(c.la, c.lb, c.lc) * g.ntile * 32L;
-        for (int k0 = 0; k0 < c.ngroup;) {
-            // one wave: as many whole groups as the stream's slice of W holds
-            int k1 = k0;
-            while (k1 < c.ngroup && c.first_chunk[k1 + 1] - c.first_chunk[k0] <= 65535 &&
-                   (c.rows[k1 + 1] - c.rows[k0]) * row <= slice)
-                ++k1;
-            if (k1 == k0)
-                return set_error(DFB_ERR_INVALID, "class (%d,%d,%d) needs %ld scratch doubles per stream, %ld given", c.la,
-                                 c.lb, c.lc, (c.rows[k0 + 1] - c.rows[k0]) * row, slice);
-            g.chunks = reinterpret_cast<const GradChunk*>(c.chunks) + c.first_chunk[k0];
-            g.nchunk = (int)(c.first_chunk[k1] - c.first_chunk[k0]);
-            g.row_base = m.row_base = (int)c.rows[k0];
-            m.groups = reinterpret_cast<const int2*>(c.groups) + k0;
-            L.ngroup = k1 - k0;
-            cudaError_t e = kInt[c.la][c.lb](L);
-            if (e != cudaSuccess) return set_cuda_error("primitive integral launch", e);
-            if (bra->b_dummy) {
-                k_prim_out2<<<dim3(c.nbra_groups, L.ngroup), 128, 0, st>>>(m, c.bra_groups, c.bra_prim0, c.la, c.la == c.lc);
-                e = cudaGetLastError();
-            } else {
-                e = kOut[c.la][c.lb](L);
+        // tiles of a wave: all of them where one group over all fits, else what does (blockIdx.z covers 65535 x 128
+        // pairs)
+        const long tiles = ((long)c.npair + 31) / 32, big = group_rows(c);
+        long step = tiles;
+        if (!bra->b_dummy) {
+            const long fit = big > 0 ? slice / (big * tile_row(c)) : tiles, grid = 65535L * (GRAD_THREADS / 32);
+            step = tiles < fit ? tiles : fit;
+            step = step < grid ? step : grid;
+        }
+        if (step < 1)
+            return set_error(DFB_ERR_INVALID, "class (%d,%d,%d) needs %ld scratch doubles per stream, %ld given", c.la, c.lb,
+                             c.lc, big * tile_row(c), slice);
+        for (long t0 = 0; t0 < tiles; t0 += step) {
+            const long p0 = 32 * t0, np = c.npair - p0 < 32 * step ? c.npair - p0 : 32 * step;
+            g.pairs = m.pairs = c.pairs + p0;
+            g.npair = m.npair = (int)np;
+            g.ntile = m.ntile = (int)((np + 31) / 32);
+            const long row = tile_row(c) * g.ntile;
+            for (int k0 = 0; k0 < c.ngroup;) {
+                // one wave: as many whole groups as the stream's slice of W holds
+                int k1 = k0;
+                while (k1 < c.ngroup && c.first_chunk[k1 + 1] - c.first_chunk[k0] <= 65535 &&
+                       (c.rows[k1 + 1] - c.rows[k0]) * row <= slice)
+                    ++k1;
+                if (k1 == k0)
+                    return set_error(DFB_ERR_INVALID, "class (%d,%d,%d) needs %ld scratch doubles per stream, %ld given",
+                                     c.la, c.lb, c.lc, (c.rows[k0 + 1] - c.rows[k0]) * row, slice);
+                g.chunks = reinterpret_cast<const GradChunk*>(c.chunks) + c.first_chunk[k0];
+                g.nchunk = (int)(c.first_chunk[k1] - c.first_chunk[k0]);
+                g.row_base = m.row_base = (int)c.rows[k0];
+                m.groups = reinterpret_cast<const int2*>(c.groups) + k0;
+                L.ngroup = k1 - k0;
+                cudaError_t e = kInt[c.la][c.lb](L);
+                if (e != cudaSuccess) return set_cuda_error("primitive integral launch", e);
+                if (bra->b_dummy) {
+                    k_prim_out2<<<dim3(c.nbra_groups, L.ngroup), 128, 0, st>>>(m, c.bra_groups, c.bra_prim0, c.la,
+                                                                              c.la == c.lc);
+                    e = cudaGetLastError();
+                } else {
+                    e = kOut[c.la][c.lb](L);
+                }
+                if (e != cudaSuccess) return set_cuda_error("group contraction launch", e);
+                count_launches(2);
+                k0 = k1;
             }
-            if (e != cudaSuccess) return set_cuda_error("group contraction launch", e);
-            count_launches(2);
-            k0 = k1;
         }
     }
     return DFB_OK;

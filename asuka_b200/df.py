@@ -39,7 +39,10 @@ _DATA = os.path.join(os.path.dirname(os.path.abspath(__file__)), "data")
 _TABLE_READY: set[int] = set()
 PRIM_SCREEN = 1e-20  # primitive-pair magnitude bound below which a pair is skipped (0 = evaluate all)
 NSTREAMS = int(os.environ.get("DFB_STREAMS", "8"))  # side streams for per-class launches (2/4/6/8 measured: 8 fastest)
-PRIM_WAVE = 1 << 23  # doubles of primitive integrals per stream and wave of a class (64 MB)
+# Doubles of primitive integrals per stream and wave of a class (8 MB; one group over 32 pairs where that is more):
+# eight streams then stay within L2.  3c integrals at 8 / 64 MB: (H2O)8 4.86 / 4.96 ms, decane 1.88 / 1.86,
+# (H2O)3 QZVP 7.85 / 7.77; scratch 71 / 535 MB
+PRIM_WAVE = 1 << 20
 # Lanes of one derivative class from which its tasks take 4 and 16 primitives: a task's set-up (rows, pair data,
 # closing sums) is shared, but too few tasks leave SMs idle (2^19 and none: (H2O)8 7.15 ms, decane 2.92;
 # 2^17 and 2^20: 6.51 and 2.48)

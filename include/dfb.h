@@ -268,6 +268,10 @@ typedef struct {
     int f32;                       /* 1: FP32 recurrence tables and accumulators per primitive (AO bra) */
 } dfb_prim_class_t;
 
+/*
+ * Doubles of scratch per stream for waves of about `target` doubles: at most target, or one group over 32 AO pairs
+ * (metric: over all primitives of the bra l) where that is more.
+ */
 long dfb_prim_scratch(const dfb_prim_class_t *cls, int ncls, long target);
 
 /*

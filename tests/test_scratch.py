@@ -96,3 +96,29 @@ def test_captured_call_outlives_larger_ones():
         torch.cuda.synchronize()
         assert torch.equal(V, V0)
     assert all(bool(torch.isnan(t).all()) for t in junk)  # the replay wrote to none of it
+
+
+@pytest.mark.parametrize("l", [(0, 0, 0), (1, 1, 2), (2, 1, 4), (4, 4, 6)])
+@pytest.mark.parametrize("npair", [1, 32, 33, 5000])
+def test_rows_stay_within_the_target(l, npair):
+    """Scratch of one class on the host: the target, unless all rows take less or one group over one tile of 32
+    pairs takes more; the pair count does not enter otherwise."""
+    import numpy as np
+
+    from asuka_b200 import _lib
+
+    if not __import__("os").path.exists(_lib.LIB_PATH):
+        pytest.skip("library not built")
+    L = _lib.lib()
+    rows = np.array([0, 5, 27, 30], dtype=np.int64)  # groups of 5, 22 and 3 primitives
+    nc = [(k + 1) * (k + 2) // 2 for k in range(10)]
+    la, lb, lc = l
+    tile = 32 * nc[lc] * sum(nc[la:la + lb + 1])
+    c = _lib.PrimClass(la, lb, lc, npair, 0, 0, 0, rows.ctypes.data, rows.ctypes.data, 3, 2, 0, 0, 0, 0)
+    for target in (1, 1 << 16, 1 << 20, 1 << 30):
+        need = L.dfb_prim_scratch(ctypes.byref(c), 1, target)
+        assert need <= max(target, 22 * tile)
+        assert need == min(max(target, 22 * tile), 30 * tile * -(-npair // 32))
+    c.bra_groups = 1  # metric: all pairs
+    need = L.dfb_prim_scratch(ctypes.byref(c), 1, 1)
+    assert need == 22 * tile * -(-npair // 32)
