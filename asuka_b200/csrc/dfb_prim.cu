@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(128) k_prim_out2(PrimOutArgs m, const int* __r
 }
 
 // Zeros for AO pairs without primitive pairs: thread = element of the pair's block, blockIdx.x = pair,
-// blockIdx.y strides over the aux functions.
+// blockIdx.y strides over the aux functions.  The index of the smaller stride runs fastest.
 __global__ void __launch_bounds__(128) k_zero_pairs(const int* __restrict__ list, const int* __restrict__ shA,
                                                     const int* __restrict__ shB, const int* __restrict__ aostart,
                                                     const int* __restrict__ nao_sh, long naux, double* __restrict__ out,
@@ -122,9 +122,10 @@ __global__ void __launch_bounds__(128) k_zero_pairs(const int* __restrict__ list
     const int pair = list[blockIdx.x];
     const int A = shA[pair], B = shB[pair];
     const int na = nao_sh[A], nb = nao_sh[B];
+    const bool p_first = sP < sN;
     for (long i = (long)blockIdx.y * blockDim.x + threadIdx.x; i < naux * na * nb; i += (long)gridDim.y * blockDim.x) {
-        const int ib = (int)(i % nb), ia = (int)((i / nb) % na);
-        const long P = i / (na * nb);
+        const long P = p_first ? i % naux : i / (na * nb);
+        const int ab = (int)(p_first ? i / naux : i % (na * nb)), ia = ab / nb, ib = ab - ia * nb;
         const long mu = aostart[A] + ia, nu = aostart[B] + ib;
         out[P * sP + mu * sM + nu * sN] = 0.0;
         out[P * sP + nu * sM + mu * sN] = 0.0;

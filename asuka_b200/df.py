@@ -43,6 +43,11 @@ NSTREAMS = int(os.environ.get("DFB_STREAMS", "8"))  # side streams for per-class
 # eight streams then stay within L2.  3c integrals at 8 / 64 MB: (H2O)8 4.86 / 4.96 ms, decane 1.88 / 1.86,
 # (H2O)3 QZVP 7.85 / 7.77; scratch 71 / 535 MB
 PRIM_WAVE = 1 << 20
+# Share of dropped elements from which a memset of the tensor is faster than zeros for the dropped blocks, whose rows
+# are one AO shell long in 'Qmn' and one aux range in 'mnQ'.  Qmn, blocks / memset: (H2O)8 share 0.18 0.85 / 0.34 ms,
+# decane 0.14 0.24 / 0.12, (H2O)3 QZVP 0.06 0.34 / 0.41, (H2O)3 TZVP 0.02 0.015 / 0.025; mnQ: 0.13 / 0.34, 0.04 / 0.12,
+# 0.08 / 0.40, 0.014 / 0.024, (H2O)5 share 0.12 0.046 / 0.088 (even at 0.07 and at 0.23 to 0.46)
+ZERO_SHARE = (1 / 16, 1 / 4)  # 'Qmn', 'mnQ'
 # Lanes of one derivative class from which its tasks take 4 and 16 primitives: a task's set-up (rows, pair data,
 # closing sums) is shared, but too few tasks leave SMs idle (2^19 and none: (H2O)8 7.15 ms, decane 2.92;
 # 2^17 and 2^20: 6.51 and 2.48)
@@ -614,11 +619,11 @@ class DFEngine:
 
     def _clear_dropped(self, X, strides, naux) -> None:
         """Zeros where the dropped shell pairs would be: their blocks alone, or the whole tensor where they are
-        a quarter of it (a block's rows are short, so its writes cost about four times their bytes)."""
+        more than ZERO_SHARE of it."""
         lst, sizes, share = self._dropped
         if not self.n_dropped_pairs:
             return
-        if share >= 0.25:
+        if share >= ZERO_SHARE[strides[0] < strides[2]]:
             X.zero_()
             return
         rc = _lib.lib().dfb_zero_pairs(ctypes.byref(self.bra_ao), _lib.ptr(lst), lst.numel(), _lib.ptr(sizes), naux,

@@ -122,3 +122,48 @@ def test_rows_stay_within_the_target(l, npair):
     c.bra_groups = 1  # metric: all pairs
     need = L.dfb_prim_scratch(ctypes.byref(c), 1, 1)
     assert need == 22 * tile * -(-npair // 32)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("share", [0.0, 1.0], ids=["memset", "blocks"])
+def test_zeros_of_dropped_pairs(monkeypatch, share):
+    """Both ways of clearing the dropped pairs leave the same integrals in both layouts, over a NaN-filled tensor
+    for the blocks of which there are some and none."""
+    import numpy as np
+
+    from asuka_b200 import basis as bm
+    from asuka_b200 import df, geometry as geo
+
+    monkeypatch.setattr(df, "ZERO_SHARE", (share, share))
+    mol = geo.water_cluster(2, 3, "ma-svp")
+    atoms = [(el, np.array(x) + 40.0 * (i >= 3)) for i, (el, x) in enumerate(mol.atoms_bohr)]  # far apart
+    eng = df.DFEngine(bm.pack_basis(atoms, mol.basis, "ao"), bm.pack_basis(atoms, mol.basis, "aux"))
+    assert eng.n_dropped_pairs
+    full = df.DFEngine(eng.ao, eng.aux, prim_screen=0.0)
+    assert not full.n_dropped_pairs
+    ref = full.int3c("Qmn")
+    for layout, back in (("Qmn", (0, 1, 2)), ("mnQ", (2, 0, 1))):
+        shape = (eng.naux, eng.nao, eng.nao) if layout == "Qmn" else (eng.nao, eng.nao, eng.naux)
+        X = torch.full(shape, float("nan"), dtype=torch.float64, device="cuda")
+        X = eng.int3c(layout, out=X).permute(back)
+        assert float((X - ref).abs().max()) <= 1e-13 * float(ref.abs().max())
+        assert float((X == 0).double().mean()) > 0.3
+
+
+@pytest.mark.parametrize("layout,share,blocks", [("Qmn", 0.05, True), ("Qmn", 0.1, False), ("Qmn", 0.2, False),
+                                                 ("mnQ", 0.1, True), ("mnQ", 0.2, True), ("mnQ", 0.3, False)])
+def test_rule_of_the_zeros(monkeypatch, layout, share, blocks):
+    """The measured crossing, about 0.07 of a 'Qmn' tensor and 0.3 of a large 'mnQ' one."""
+    from asuka_b200 import _lib, df
+
+    calls = []
+    fake = type("L", (), {"dfb_zero_pairs": lambda self, *a: calls.append(a) or 0})()
+    monkeypatch.setattr(_lib, "lib", lambda: fake)
+    monkeypatch.setattr(df, "_stream", lambda: 0)
+    eng = df.DFEngine.__new__(df.DFEngine)
+    eng.n_dropped_pairs, eng.bra_ao = 3, _lib.Bra()
+    lst = torch.zeros(3, dtype=torch.int32)
+    eng._dropped = (lst, lst, share)
+    X = torch.ones(8)
+    eng._clear_dropped(X, (16, 4, 1) if layout == "Qmn" else (1, 32, 8), 8)
+    assert bool(calls) == blocks and bool((X == 0).all()) != blocks
