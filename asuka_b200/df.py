@@ -155,6 +155,11 @@ def _as_soa(b) -> BasisCartSoA:
     return b if isinstance(b, BasisCartSoA) else from_reference_like(b)
 
 
+def _with_aux(classes, byl):
+    """Class entries with their aux shells: their own, or those of the block (``byl``) where they name none."""
+    return [(la, lb, lc, pairs, byl[lc] if auxs is None else auxs) for la, lb, lc, pairs, auxs in classes]
+
+
 class DFEngine:
     """Device-side state of the DF Rys integrals for one (AO, aux) basis pair."""
 
@@ -209,23 +214,12 @@ class DFEngine:
         self.axs = _lib.AuxSide(*[_lib.ptr(t) for t in (self.ax_cxyz, self.ax_pstart, self.ax_nprim, self.ax_exp,
                                                         self.ax_coef, self.ax_rexp, self.ax_aostart, self.ax_atom)])
         self._classes2c = None
-        self._epoch = 0
         self.groups = AuxGroups(aux, np.arange(aux.nshell), dev, self.ax_cxyz, self.ax_aostart, self.ax_atom)
         self._scratch = scratch if scratch is not None else ScratchHolder()
         self._build_ao_pairs(ao.shell_cxyz)
         self._build_pair_tables()
 
     # ------------------------------------------------------------ class lists
-    @property
-    def classes3c(self):
-        """(la, lb, lc, AO pair list, aux shell list) per angular class; assigning a list drops the launch plans."""
-        return self._classes3c
-
-    @classes3c.setter
-    def classes3c(self, classes) -> None:
-        self._classes3c = classes
-        self._epoch += 1
-
     @property
     def classes2c(self):
         """Metric classes of the shell-by-shell kernels: (lP, lQ, P list, Q list) over the unordered aux shell
@@ -352,8 +346,11 @@ class DFEngine:
                                     self.ao_aostart, self.ao_atom)], 0)
         # dropped shell pairs write nothing: outputs are zero-filled first when any exist
         self.n_dropped_pairs = int((~live).sum())
-        self.classes3c = [(a, b, c, pairs, auxs) for (a, b), pairs in ((k, di(h)) for k, h in ph.items())
-                          for c, auxs in self.aux_by_l.items()]  # (la, lb, lc, pairs tensor, aux tensor)
+        # (la, lb, lc, AO pair list, aux shell list) per angular class.  A program may assign or edit the list: entries
+        # with lists of their own run on the shell kernels (_make_plan)
+        self._pairs3c = {key: di(h) for key, h in ph.items()}
+        self.classes3c = [(a, b, c, pairs, auxs) for (a, b), pairs in self._pairs3c.items()
+                          for c, auxs in self.aux_by_l.items()]
         self._aux_blocks_n = None
 
     # ------------------------------------------------------------ helpers
@@ -555,41 +552,56 @@ class DFEngine:
         return grad
 
     # ------------------------------------------------------------ group-kernel routes
-    def _plan(self, kind: str, groups: AuxGroups, precision: str):
+    def _plan(self, kind: str, groups: AuxGroups, precision: str, block: bool = False):
         """Launch plan of one contraction ('int', 'der', or with '2' for the metric) over ``groups``: (ctypes
-        class array, its length, the classes left to the shell-by-shell kernels as (la, lb, lc, pairs)),
-        kept with the groups until the class lists change.
+        class array, its length, the classes left to the shell-by-shell kernels as (la, lb, lc, pairs, auxs),
+        scratch), kept with the groups while the class list holds the same entries.
 
         The group kernels (``dfb_prim_integrals``, ``dfb_grad_contract``) take every class with bra l <= 4
         (the metric: l <= 8).  Left on ``dfb_rys_*_prec``: AO shells above g, 'mixed_all' (which measures the
         FP32 shell kernels) and the generic-kernel switch DFB_DISABLE_TMPL."""
         shells = precision == "mixed_all" or bool(os.environ.get("DFB_DISABLE_TMPL"))
         f32 = frozenset(mixed_class_table().get("int3c", ())) if precision == "mixed" and kind == "int" else None
-        key = (kind, shells, f32, self._epoch)
-        plan = groups.plans.get(key)
-        if plan is None:
-            if len(groups.plans) > 16:
-                groups.plans.clear()
-            plan = groups.plans[key] = self._make_plan(kind, groups, shells, f32 or ())
+        key = (kind, shells, f32, block)
+        now = () if kind.endswith("2") else self.classes3c
+        known = groups.plans.get(key)
+        if known is not None:
+            entries, plan = known
+            if len(entries) == len(now) and all(a is b for a, b in zip(entries, now)):
+                return plan
+        if len(groups.plans) > 16:
+            groups.plans.clear()
+        plan = self._make_plan(kind, groups, shells, f32 or (), block)
+        groups.plans[key] = (tuple(now), plan)
         return plan
 
-    def _make_plan(self, kind: str, groups: AuxGroups, shells: bool, f32):
+    def _make_plan(self, kind: str, groups: AuxGroups, shells: bool, f32, block: bool):
         metric, deriv = kind.endswith("2"), kind.startswith("der")
         if metric:
             ls = sorted(groups.by_l)
-            classes = [(lp, 0, lq, groups.prim_ids(lp)) for lp in ls for lq in ls if lq <= lp]
-        else:
-            classes = list({(la, lb, lc): (la, lb, lc, pairs) for la, lb, lc, pairs, _a in self._classes3c
-                            if lc in groups.by_l}.values())
+            classes = [(lp, 0, lq, groups.prim_ids(lp), None) for lp in ls for lq in ls if lq <= lp]
+        elif not block:
+            classes = self.classes3c
+        else:  # the block's aux shells with the pairs of the class's first entry
+            first: dict = {}
+            for la, lb, lc, pairs, _auxs in self.classes3c:
+                if lc in groups.by_l:
+                    first.setdefault((la, lb, lc), (la, lb, lc, pairs, None))
+            classes = list(first.values())
         L = _lib.lib()
-        new = [c for c in classes if not shells and L.dfb_grad_supported(*c[:3], int(metric))]
-        old = [c for c in classes if c not in new]
+        new, old = [], []
+        for c in classes:
+            la, lb, lc, pairs, auxs = c
+            # the group kernels evaluate whole classes: all pairs of (la, lb) against all aux shells of lc
+            whole = metric or (pairs is self._pairs3c.get((la, lb)) and (auxs is None or auxs is self.aux_by_l.get(lc)))
+            group = whole and not shells and L.dfb_grad_supported(la, lb, lc, int(metric))
+            (new if group else old).append(c)
         # the longest single tasks (high bra l, few pairs) first: the numerous low classes fill in behind them
         new.sort(key=lambda c: -(c[0] + c[1]))
         nprim = {l: hi - lo for l, (lo, hi) in groups.prims.items()}
         arr = ((_lib.GradClass if deriv else _lib.PrimClass) * max(len(new), 1))()
         p = _lib.ptr
-        for i, (la, lb, lc, pairs) in enumerate(new):
+        for i, (la, lb, lc, pairs, _auxs) in enumerate(new):
             if deriv and not metric:
                 pairs = self._seg_lists[la, lb]
             n = int(pairs.numel())
@@ -610,11 +622,12 @@ class DFEngine:
         return arr, len(new), old, per
 
     def _int3c_work(self, X, strides, precision, groups=None, axs=None, byl=None):
+        block = groups is not None
         groups, axs, byl = groups or self.groups, axs or self.axs, byl or self.aux_by_l
-        arr, n, old, per = self._plan("int", groups, precision)
+        arr, n, old, per = self._plan("int", groups, precision, block)
         pc = _prec_code(precision)
-        rest = [(la, lb, lc, self.ps_ao, axs, pairs, byl[lc], pairs.numel() * byl[lc].numel(), -pairs.numel(), 0, X,
-                 strides, pc) for la, lb, lc, pairs in old]
+        rest = [(la, lb, lc, self.ps_ao, axs, pairs, auxs, pairs.numel() * auxs.numel(), -pairs.numel(), 0, X, strides, pc)
+                for la, lb, lc, pairs, auxs in _with_aux(old, byl)]
         return self.bra_ao, groups, arr, n, per, X, strides, rest
 
     def _clear_dropped(self, X, strides, naux) -> None:
@@ -639,11 +652,12 @@ class DFEngine:
         return self.groups.bra, self.groups, arr, n, per, V, s, rest
 
     def _deriv3c_work(self, bar, strides, grad, precision, groups=None, axs=None, byl=None):
+        block = groups is not None
         groups, axs, byl = groups or self.groups, axs or self.axs, byl or self.aux_by_l
-        arr, n, old, _per = self._plan("der", groups, precision)
+        arr, n, old, _per = self._plan("der", groups, precision, block)
         pc = _prec_code(precision)
-        rest = [(la, lb, lc, self.ps_ao, axs, pairs, byl[lc], pairs.numel() * byl[lc].numel(), -pairs.numel(), 0, bar,
-                 strides, grad, pc) for la, lb, lc, pairs in old]
+        rest = [(la, lb, lc, self.ps_ao, axs, pairs, auxs, pairs.numel() * auxs.numel(), -pairs.numel(), 0, bar, strides,
+                 grad, pc) for la, lb, lc, pairs, auxs in _with_aux(old, byl)]
         return self.bra_seg, groups, arr, n, bar, strides, rest
 
     def _deriv2c_work(self, bar, grad, precision):
