@@ -16,6 +16,8 @@ import torch
 from . import _lib
 
 NQ = (1, 4, 16)  # largest primitive counts of a task: one where tasks are few, more where set-up is worth sharing
+# first bra entries of the chunk lists (AuxGroups.chunks) by primitive count: integrals take one primitive per task
+PLO = {1: ("all", "own", "after"), 4: ("all", "after"), 16: ("all", "after")}
 
 
 class DevicePool:
@@ -103,17 +105,20 @@ class AuxGroups:
             n, p0 = inf[:, 2], inf[:, 1]
             lo = self.prims[l][0]
             rows = np.concatenate([[0], np.cumsum(n)])
-            out["g", l] = np.stack([np.asarray(gs), rows[:-1]], axis=1)
-            out["i", l] = np.asarray(gs)
+            inf0 = np.asarray(gs)
+            out["g", l] = np.stack([inf0, rows[:-1]], axis=1)
+            out["i", l] = inf0
             out["p", l] = np.arange(*self.prims[l])
             for nq in NQ:
                 cnt = -(-n // nq)  # chunks per group
                 first = np.concatenate([[0], np.cumsum(cnt)])
                 g = np.repeat(np.arange(len(gs)), cnt)
                 k = (np.arange(first[-1]) - first[g]) * nq
-                base = (np.asarray(gs)[g], p0[g] + k, np.minimum(nq, n[g] - k), rows[g] + k)
-                for plo, v in (("all", np.zeros_like(k)), ("own", p0[g] - lo), ("after", p0[g] + n[g] - lo)):
-                    out["c", l, nq, plo] = np.stack([*base, v], axis=1)
+                base = np.stack([inf0[g], p0[g] + k, np.minimum(nq, n[g] - k), rows[g] + k, np.zeros_like(k)], axis=1)
+                for plo in PLO[nq]:
+                    out["c", l, nq, plo] = lst = base if plo == "all" else base.copy()
+                    if plo != "all":
+                        lst[:, 4] = (p0 - lo if plo == "own" else p0 + n - lo)[g]
                 self._rows[l, nq] = (rows, first)
         return out
 

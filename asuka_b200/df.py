@@ -422,6 +422,9 @@ class DFEngine:
                 s1 += 1
             p0 = int(aux.shell_ao_start[s0])
             p1 = p0 + int(tot)
+            if s1 - s0 == aux.nshell and p0 == 0:  # one block: the engine's own lists
+                blocks.append((p0, p1, (self.axs, self.ax_aostart, self.aux_by_l, self.groups)))
+                break
             shifted = torch.as_tensor(aux.shell_ao_start.astype(np.int32) - p0, device=self.device)
             axb = _lib.AuxSide(*[_lib.ptr(t) for t in (self.ax_cxyz, self.ax_pstart, self.ax_nprim, self.ax_exp,
                                                        self.ax_coef, self.ax_rexp, shifted, self.ax_atom)])

@@ -98,3 +98,16 @@ def test_edited_lists_match_the_shell_kernels(monkeypatch, name):
     old = run()
     for i, (a, b) in enumerate(zip(new, old)):
         assert float((a - b).abs().max()) <= (4e-13 if i < 2 else 1e-11) * float(b.abs().max()), i
+
+
+@pytest.mark.gpu
+def test_one_block_takes_the_engines_lists():
+    """A block that holds the whole aux basis shares the engine's groups (nothing is built for it twice), and is
+    bit for bit the whole tensor; smaller blocks have groups of their own."""
+    from asuka_b200 import df
+
+    eng = df.DFEngine(*_bases())
+    ((p0, p1, blk),) = eng.aux_blocks(10 ** 6)
+    assert (p0, p1) == (0, eng.naux) and blk[3] is eng.groups
+    assert torch.equal(eng.int3c_block(blk, p0, p1), eng.int3c("Qmn"))
+    assert all(b[2][3] is not eng.groups for b in eng.aux_blocks(50))
