@@ -125,10 +125,9 @@ def _prec_code(precision: str) -> int:
 @functools.lru_cache(maxsize=1)
 def mixed_class_table() -> dict:
     """Angular classes whose FP32-component kernels the mixed mode uses, per kind, as sets of
-    (la, lb, lc).  Written by ``asuka_b200.tune_precision`` from the measured first-order energy and
-    gradient errors of every class (FP32 against FP64 kernels); classes not listed run in FP64 in
-    mixed mode too.  The mixed mode reads 'int3c': its derivative contractions run on the FP64 group
-    kernels, which are faster than the FP32 shell kernels ('deriv3c' and 'deriv2c' were measured for those)."""
+    (la, lb, lc): the 3c integrals ('int3c').  Written by ``asuka_b200.tune_precision`` from the first-order
+    energy and gradient errors and the times of every class on the group kernels; classes not listed, the metric
+    and the derivative contractions run in FP64 in mixed mode too."""
     p = os.path.join(_DATA, "class_precision.json")
     if not os.path.exists(p):
         return {}
@@ -136,7 +135,7 @@ def mixed_class_table() -> dict:
 
     with open(p) as f:
         t = json.load(f)
-    return {k: {tuple(int(v) for v in c) for c in t.get(k, [])} for k in ("int3c", "deriv3c", "deriv2c")}
+    return {k: {tuple(int(v) for v in c) for c in t.get(k, [])} for k in ("int3c",)}
 
 
 def _class_prec(code: int, kind: str, la: int, lb: int, lc: int) -> int:

@@ -257,10 +257,11 @@ def df_energy_grad_streamed(engine: DFEngine, Cw: torch.Tensor, aux_block: int =
     block's derivative integrals (the streamed analogue of
     ``asuka/hf/df_jk_streamed.py:167-325``, with the gradient recomputing the integrals
     instead of reading a stored B).  The largest buffer is Y/W (naux x nao x nocc)
-    instead of the 3c tensor (naux x nao^2).  ``precision='mixed'`` evaluates the
-    integrals and their derivatives with FP32 recurrence tables and accumulators and
-    runs the exchange update K as a split-BF16 tensor-core GEMM; the metric solves stay
-    FP64 unless ``mixed_solve`` (split-BF16 product with L^-1) is asked for.
+    instead of the 3c tensor (naux x nao^2).  ``precision='mixed'`` evaluates the 3c
+    integrals of the classes in ``df.mixed_class_table`` with FP32 recurrence tables and
+    accumulators and runs the exchange update K as a split-BF16 tensor-core GEMM; the
+    derivative integrals are FP64, and so are the metric solves unless ``mixed_solve``
+    (split-BF16 product with L^-1) is asked for.
     Returns (E, grad (natm, 3), K).
     """
     nao, naux = engine.nao, engine.naux

@@ -109,8 +109,8 @@ class DFGradContractionContext:
     # ------------------------------------------------------------ contractions
     def contract_device(self, *, B_ao: Any, bar_L_ao: Any, aux_block_naux: int = 128,
                         precision: str = "fp64") -> torch.Tensor:
-        """(natm, 3) device gradient; ``precision='mixed'`` runs the derivative integrals with FP32
-        recurrences and accumulators (``DFB_PREC_MIXED``); the adjoints stay FP64."""
+        """(natm, 3) device gradient.  The derivative integrals of ``precision='mixed'`` run in FP64, as all else
+        here does ('mixed_all': on the FP32 shell kernels, for measurements)."""
         dev = self.engine.device
         B = torch.as_tensor(B_ao, dtype=torch.float64, device=dev)
         barL = torch.as_tensor(bar_L_ao, dtype=torch.float64, device=dev)

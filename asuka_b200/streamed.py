@@ -10,8 +10,8 @@ density for J (UHF alpha/beta), with the same argument meaning.  Per call:
 * d = V^-1 rho, W_j = L^-1 Y_j (block substitution), K_j = sum_Q W_jQ W_jQ^T;
 * pass 2: J = sum_P d_P X_P with the blocks recomputed.
 
-``precision='mixed'`` evaluates the integrals with FP32 recurrence tables and
-accumulators (``DFB_PREC_MIXED``) and the exchange update as a split-BF16
+``precision='mixed'`` evaluates the integrals of the classes in ``df.mixed_class_table``
+with FP32 recurrence tables and accumulators and the exchange update as a split-BF16
 tensor-core GEMM; the SCF finishes with FP64 iterations.
 
 Outputs are symmetric FP64 device tensors.

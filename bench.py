@@ -418,7 +418,7 @@ def run_gpu(args) -> dict | None:
         "vs_baseline": None, "dtype": "f64", "data": "synthetic (seeded geometry; basis tables from the reference)",
         "config": {"workload": WORKLOAD, "nao": nao, "naux": naux,
                    "precision": "mixed: FP32-component Rys kernels for the angular classes the precision table admits "
-                                f"({mixed_counts}, chosen by asuka_b200.tune_precision within 2.5e-7 Eh and 2.5e-7 "
+                                f"({mixed_counts}, chosen by asuka_b200.tune_precision within 2.5e-8 Eh and 2.5e-8 "
                                 "Eh/bohr), split-BF16 tcgen05 exchange update; FP64 roots/weights, metric, solves, derivative contractions, "
                                 "Y = X Cw, adjoints, energy and gradient accumulation",
                    "l2": "working set (3c tensor 2.5 GB) > L2 126 MB", "replicas": world if world > 1 else None},
