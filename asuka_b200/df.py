@@ -154,6 +154,47 @@ def _as_soa(b) -> BasisCartSoA:
     return b if isinstance(b, BasisCartSoA) else from_reference_like(b)
 
 
+class _PairStatic:
+    """What the AO pair lists of every geometry share: the primitive pairs of all shell pairs (owner, index within
+    it, and the factors of their magnitude bound), the angular class of each shell pair, and the pairs by
+    (class, A, B)."""
+
+    def __init__(self, ao: BasisCartSoA, sp):
+        npr = sp.sp_npair.astype(np.int64)
+        self.owner = np.repeat(np.arange(sp.nsp), npr)
+        self.loc = (np.arange(self.owner.size) - np.repeat(sp.sp_pair_start[:-1].astype(np.int64), npr)).astype(np.int32)
+        A, B = sp.sp_A[self.owner], sp.sp_B[self.owner]
+        nb = ao.shell_nprim[B]
+        pa = ao.shell_prim_start[A] + self.loc // nb
+        pb = ao.shell_prim_start[B] + self.loc % nb
+        a, b = ao.prim_exp[pa], ao.prim_exp[pb]
+        p = a + b
+        self.coef = np.abs(ao.prim_coef[pa] * ao.prim_coef[pb])
+        self.mexp = -a * b / p
+        self.power = (np.pi / p) ** 1.5
+        la, lb = ao.shell_l[sp.sp_A].astype(np.int64), ao.shell_l[sp.sp_B].astype(np.int64)
+        self.classes, cls = np.unique(la * 16 + lb, return_inverse=True)
+        self.cls = cls.astype(np.int64)
+        self.order = np.lexsort((sp.sp_B, sp.sp_A, self.cls))
+
+
+def _stable_order(key: np.ndarray) -> np.ndarray:
+    """argsort of an integer key, equal keys in their order (16-bit keys sort by radix)."""
+    if key.size and -32768 <= key.min() and key.max() <= 32767:
+        key = key.astype(np.int16)
+    return np.argsort(key, kind="stable")
+
+
+def _split_classes(st: _PairStatic, cls: np.ndarray, items: np.ndarray, pool: DevicePool) -> dict:
+    """(la, lb) -> pool handle of the items of that class; ``items`` and their classes come ordered by class."""
+    out = {}
+    cut = np.searchsorted(cls, np.arange(len(st.classes) + 1))
+    for i, code in enumerate(st.classes.tolist()):
+        if cut[i + 1] > cut[i]:
+            out[code // 16, code % 16] = pool.add(items[cut[i]:cut[i + 1]])
+    return out
+
+
 def _with_aux(classes, byl):
     """Class entries with their aux shells: their own, or those of the block (``byl``) where they name none."""
     return [(la, lb, lc, pairs, byl[lc] if auxs is None else auxs) for la, lb, lc, pairs, auxs in classes]
@@ -215,6 +256,7 @@ class DFEngine:
         self._classes2c = None
         self.groups = AuxGroups(aux, np.arange(aux.nshell), dev, self.ax_cxyz, self.ax_aostart, self.ax_atom)
         self._scratch = scratch if scratch is not None else ScratchHolder()
+        self._pair_static = _PairStatic(ao, self.sp)
         self._build_ao_pairs(ao.shell_cxyz)
         self._build_pair_tables()
 
@@ -277,63 +319,49 @@ class DFEngine:
         reference evaluates every pair (``asuka/cueri/gpu.py:1833-1834``); ``prim_screen=0``
         reproduces that exactly.
         """
-        ao, sp = self.ao, self.sp
-        npr = sp.sp_npair.astype(np.int64)
-        owner = np.repeat(np.arange(sp.nsp), npr)
-        loc = (np.arange(owner.size) - np.repeat(sp.sp_pair_start[:-1].astype(np.int64), npr)).astype(np.int32)
-        A = sp.sp_A[owner]
-        B = sp.sp_B[owner]
-        nb = ao.shell_nprim[B]
-        pa = ao.shell_prim_start[A] + loc // nb
-        pb = ao.shell_prim_start[B] + loc % nb
+        sp, st = self.sp, self._pair_static
         if self.prim_screen > 0.0:
-            a, b = ao.prim_exp[pa], ao.prim_exp[pb]
-            R2 = ((shell_cxyz[A] - shell_cxyz[B]) ** 2).sum(1)
-            p = a + b
-            bound = np.abs(ao.prim_coef[pa] * ao.prim_coef[pb]) * np.exp(-a * b / p * R2) * (np.pi / p) ** 1.5
+            R2 = ((shell_cxyz[sp.sp_A] - shell_cxyz[sp.sp_B]) ** 2).sum(1)
+            bound = st.coef * np.exp(st.mexp * R2[st.owner]) * st.power
             keep = bound >= self.prim_screen
+            kept_owner, kept_loc = st.owner[keep], st.loc[keep]
         else:
-            keep = np.ones(owner.size, dtype=bool)
-        kept_owner = owner[keep]
-        cnt = np.bincount(kept_owner, minlength=sp.nsp).astype(np.int32)
+            kept_owner, kept_loc = st.owner, st.loc
+        cnt = np.bincount(kept_owner, minlength=sp.nsp)
         start = np.zeros(sp.nsp, dtype=np.int64)
         np.cumsum(cnt[:-1], out=start[1:])
-        la = ao.shell_l[sp.sp_A]
-        lb = ao.shell_l[sp.sp_B]
         live = cnt > 0
         pool = DevicePool(np.int32)
-        hs = [pool.add(a) for a in (start, cnt, kept_owner, loc[keep])]
-        ph = {}
-        for a in np.unique(la):
-            for b in np.unique(lb):
-                sel = np.nonzero((la == a) & (lb == b) & live)[0]
-                if sel.size:
-                    # pairs by decreasing primitive-pair count: with the aux-major task
-                    # grid a warp walks pairs of similar cost against one aux shell.  Equal
-                    # counts by (A, B): neighbouring pairs then read and write neighbouring
-                    # columns of one 3c row
-                    sel = sel[np.lexsort((sp.sp_B[sel], sp.sp_A[sel], -cnt[sel]))]
-                    ph[int(a), int(b)] = pool.add(sel)
-        # derivative bra entries: segments of at most SEG_PRIMS primitive pairs (their contributions add)
-        nseg = -(-cnt.astype(np.int64) // SEG_PRIMS)
-        seg_pair = np.repeat(np.arange(sp.nsp), nseg)
+        hs = [pool.add(a) for a in (start, cnt, kept_owner, kept_loc)]
+        # pairs of a class by decreasing primitive-pair count: with the aux-major task grid a warp walks pairs of
+        # similar cost against one aux shell.  Equal counts by (A, B): neighbouring pairs then read and write
+        # neighbouring columns of one 3c row
+        order = st.order[live[st.order]]
+        top = int(cnt.max(initial=0)) + 1
+        order = order[_stable_order(st.cls[order] * top - cnt[order])]
+        ph = _split_classes(st, st.cls[order], order, pool)
+        # derivative bra entries: segments of at most SEG_PRIMS primitive pairs (their contributions add), by class,
+        # decreasing length and (A, B)
+        nseg = -(-cnt[st.order] // SEG_PRIMS)
+        seg_pair = np.repeat(st.order, nseg)
         k = np.arange(seg_pair.size) - np.repeat(np.cumsum(nseg) - nseg, nseg)
         seg_n = np.minimum(SEG_PRIMS, cnt[seg_pair] - SEG_PRIMS * k)
         gs = [pool.add(a) for a in (sp.sp_A[seg_pair], sp.sp_B[seg_pair], start[seg_pair] + SEG_PRIMS * k, seg_n)]
-        gh = {}
-        for (a, b) in ph:
-            sel = np.nonzero((la[seg_pair] == a) & (lb[seg_pair] == b))[0]
-            gh[a, b] = pool.add(sel[np.lexsort((k[sel], sp.sp_B[seg_pair[sel]], sp.sp_A[seg_pair[sel]], -seg_n[sel]))])
-        hz, hn = pool.add(np.nonzero(~live)[0]), pool.add((ao.shell_l + 1) * (ao.shell_l + 2) // 2)
+        seg_cls = st.cls[seg_pair]
+        order = _stable_order(seg_cls * (SEG_PRIMS + 1) - seg_n)
+        gh = _split_classes(st, seg_cls[order], order, pool)
+        ao = self.ao
         size = (ao.shell_l.astype(np.int64) + 1) * (ao.shell_l + 2) // 2
-        dropped = float((size[sp.sp_A] * size[sp.sp_B])[~live].sum()) * 2.0 / max(ao.nao, 1) ** 2
+        gone = np.nonzero(~live)[0]
+        hz, hn = pool.add(gone), pool.add(size)
+        dropped = float((size[sp.sp_A[gone]] * size[sp.sp_B[gone]]).sum()) * 2.0 / max(ao.nao, 1) ** 2
         di = pool.upload(self.device)
         self.sp_pstart, self.sp_npair, self.pp_sp, self.pp_local = (di(h) for h in hs)
         self._dropped = (di(hz), di(hn), dropped)  # pairs without primitives, shell sizes, their share of a 3c row
         self._segs = tuple(di(h) for h in gs)
         self._seg_lists = {key: di(h) for key, h in gh.items()}
-        self.n_prim_pairs = int(keep.sum())
-        self.n_prim_pairs_total = int(owner.size)
+        self.n_prim_pairs = int(kept_owner.size)
+        self.n_prim_pairs_total = int(st.owner.size)
         self.pt = torch.empty((7, max(self.n_prim_pairs, 1)), dtype=torch.float64, device=self.device)
         self.prec = torch.empty((max(self.n_prim_pairs, 1), 8), dtype=torch.float64, device=self.device)
         p = _lib.ptr
@@ -344,7 +372,7 @@ class DFEngine:
             *[_lib.ptr(t) for t in (self.sp_A, self.sp_B, self.sp_pstart, self.sp_npair, *self.pt, self.ao_cxyz,
                                     self.ao_aostart, self.ao_atom)], 0)
         # dropped shell pairs write nothing: outputs are zero-filled first when any exist
-        self.n_dropped_pairs = int((~live).sum())
+        self.n_dropped_pairs = int(gone.size)
         # (la, lb, lc, AO pair list, aux shell list) per angular class.  A program may assign or edit the list: entries
         # with lists of their own run on the shell kernels (_make_plan)
         self._pairs3c = {key: di(h) for key, h in ph.items()}
