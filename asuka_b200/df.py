@@ -154,6 +154,16 @@ def _as_soa(b) -> BasisCartSoA:
     return b if isinstance(b, BasisCartSoA) else from_reference_like(b)
 
 
+# dfb_grad_class_t and dfb_prim_class_t, filled as NumPy records
+_GRAD_CLASS = np.dtype([(n, "u8" if t is ctypes.c_void_p else "i4") for n, t in _lib.GradClass._fields_], align=True)
+_PRIM_CLASS = np.dtype([(n, "u8" if t is ctypes.c_void_p else "i4") for n, t in _lib.PrimClass._fields_], align=True)
+
+
+@functools.lru_cache(maxsize=4096)
+def _group_class(la: int, lb: int, lc: int, metric: bool) -> bool:
+    return bool(_lib.lib().dfb_grad_supported(la, lb, lc, int(metric)))
+
+
 class _PairStatic:
     """What the AO pair lists of every geometry share: the primitive pairs of all shell pairs (owner, index within
     it, and the factors of their magnitude bound), the angular class of each shell pair, and the pairs by
@@ -256,6 +266,7 @@ class DFEngine:
         self._classes2c = None
         self.groups = AuxGroups(aux, np.arange(aux.nshell), dev, self.ax_cxyz, self.ax_aostart, self.ax_atom)
         self._scratch = scratch if scratch is not None else ScratchHolder()
+        self._aux_blocks_n = None  # blocks of the aux basis (aux_blocks), which hold for every geometry
         self._pair_static = _PairStatic(ao, self.sp)
         self._build_ao_pairs(ao.shell_cxyz)
         self._build_pair_tables()
@@ -378,7 +389,6 @@ class DFEngine:
         self._pairs3c = {key: di(h) for key, h in ph.items()}
         self.classes3c = [(a, b, c, pairs, auxs) for (a, b), pairs in self._pairs3c.items()
                           for c, auxs in self.aux_by_l.items()]
-        self._aux_blocks_n = None
 
     # ------------------------------------------------------------ helpers
     def _build_pair_tables(self) -> None:
@@ -438,30 +448,35 @@ class DFEngine:
         if getattr(self, "_aux_blocks_n", None) == max_naux:
             return self._aux_blocks
         aux = self.aux
-        nc = np.array([ncart(int(l)) for l in aux.shell_l])
-        blocks = []
+        nc = [ncart(l) for l in aux.shell_l.tolist()]
+        cuts = []  # (first shell, one past the last, functions)
         s0 = 0
         while s0 < aux.nshell:
-            s1 = s0
-            tot = 0
+            s1, tot = s0, 0
             while s1 < aux.nshell and (tot + nc[s1] <= max_naux or s1 == s0):
                 tot += nc[s1]
                 s1 += 1
-            p0 = int(aux.shell_ao_start[s0])
-            p1 = p0 + int(tot)
-            if s1 - s0 == aux.nshell and p0 == 0:  # one block: the engine's own lists
-                blocks.append((p0, p1, (self.axs, self.ax_aostart, self.aux_by_l, self.groups)))
-                break
-            shifted = torch.as_tensor(aux.shell_ao_start.astype(np.int32) - p0, device=self.device)
-            axb = _lib.AuxSide(*[_lib.ptr(t) for t in (self.ax_cxyz, self.ax_pstart, self.ax_nprim, self.ax_exp,
-                                                       self.ax_coef, self.ax_rexp, shifted, self.ax_atom)])
-            byl = {}
-            for l in np.unique(aux.shell_l[s0:s1]):
-                idx = s0 + np.nonzero(aux.shell_l[s0:s1] == l)[0]
-                byl[int(l)] = torch.as_tensor(idx.astype(np.int32), device=self.device)
-            groups = AuxGroups(aux, np.arange(s0, s1), self.device, self.ax_cxyz, shifted, self.ax_atom)
-            blocks.append((p0, p1, (axb, shifted, byl, groups)))
+            cuts.append((s0, s1, tot))
             s0 = s1
+        p0s = [int(aux.shell_ao_start[s0]) for s0, _s1, _t in cuts]
+        if len(cuts) == 1 and p0s[0] == 0:  # one block: the engine's own lists
+            blocks = [(0, cuts[0][2], (self.axs, self.ax_aostart, self.aux_by_l, self.groups))]
+        else:
+            pool = DevicePool(np.int32)
+            hs, hl = [], []
+            for (s0, s1, _t), p0 in zip(cuts, p0s):
+                hs.append(pool.add(aux.shell_ao_start - p0))
+                l = aux.shell_l[s0:s1]
+                hl.append({int(v): pool.add(s0 + np.nonzero(l == v)[0]) for v in np.unique(l)})
+            di = pool.upload(self.device)
+            shifted = [di(h) for h in hs]
+            groups = AuxGroups.blocks(aux, self.groups.shell_ids, [np.arange(s0, s1) for s0, s1, _t in cuts], self.device,
+                                      self.ax_cxyz, shifted, self.ax_atom)
+            blocks = []
+            for (s0, s1, tot), p0, sh, hb, gr in zip(cuts, p0s, shifted, hl, groups):
+                axb = _lib.AuxSide(*[_lib.ptr(t) for t in (self.ax_cxyz, self.ax_pstart, self.ax_nprim, self.ax_exp,
+                                                           self.ax_coef, self.ax_rexp, sh, self.ax_atom)])
+                blocks.append((p0, p0 + tot, (axb, sh, {v: di(h) for v, h in hb.items()}, gr)))
         self._aux_blocks, self._aux_blocks_n = blocks, max_naux
         return blocks
 
@@ -608,47 +623,50 @@ class DFEngine:
     def _make_plan(self, kind: str, groups: AuxGroups, shells: bool, f32, block: bool):
         metric, deriv = kind.endswith("2"), kind.startswith("der")
         if metric:
-            ls = sorted(groups.by_l)
-            classes = [(lp, 0, lq, groups.prim_ids(lp), None) for lp in ls for lq in ls if lq <= lp]
+            ls = sorted(groups.fam)
+            classes = [(lp, 0, lq, None, None) for lp in ls for lq in ls if lq <= lp]
         elif not block:
             classes = self.classes3c
         else:  # the block's aux shells with the pairs of the class's first entry
             first: dict = {}
             for la, lb, lc, pairs, _auxs in self.classes3c:
-                if lc in groups.by_l:
+                if lc in groups.fam:
                     first.setdefault((la, lb, lc), (la, lb, lc, pairs, None))
             classes = list(first.values())
-        L = _lib.lib()
         new, old = [], []
         for c in classes:
             la, lb, lc, pairs, auxs = c
             # the group kernels evaluate whole classes: all pairs of (la, lb) against all aux shells of lc
             whole = metric or (pairs is self._pairs3c.get((la, lb)) and (auxs is None or auxs is self.aux_by_l.get(lc)))
-            group = whole and not shells and L.dfb_grad_supported(la, lb, lc, int(metric))
-            (new if group else old).append(c)
+            (new if whole and not shells and _group_class(la, lb, lc, metric) else old).append(c)
         # the longest single tasks (high bra l, few pairs) first: the numerous low classes fill in behind them
         new.sort(key=lambda c: -(c[0] + c[1]))
-        nprim = {l: hi - lo for l, (lo, hi) in groups.prims.items()}
-        arr = ((_lib.GradClass if deriv else _lib.PrimClass) * max(len(new), 1))()
-        p = _lib.ptr
-        for i, (la, lb, lc, pairs, _auxs) in enumerate(new):
-            if deriv and not metric:
-                pairs = self._seg_lists[la, lb]
-            n = int(pairs.numel())
+        if metric:
+            bra = {(l, 0): groups.prim_ids(l) for l in groups.fam}
+        else:
+            lists = self._seg_lists if deriv else self._pairs3c
+            bra = {k: (_lib.ptr(v), int(v.numel())) for k, v in lists.items()}
+        recs = []
+        for la, lb, lc, _pairs, _auxs in new:
+            pairs, n = bra[la, lb]
+            same = metric and la == lc
             if deriv:
-                lanes = n * nprim[lc] * ((la + lb + lc + 1) // 2 + 1)
+                lo, hi = groups.prims[lc]
+                lanes = n * (hi - lo) * ((la + lb + lc + 1) // 2 + 1)
                 nq = 16 if lanes >= GRAD_BIG else 4 if lanes >= GRAD_THREADS else 1
-                chunks = groups.chunks(lc, nq, "after" if metric and la == lc else "all")
-                arr[i] = _lib.GradClass(la, lb, lc, n, p(pairs), p(chunks), chunks.shape[0], nq)
+                recs.append((la, lb, lc, n, pairs, *groups.chunk_range(lc, nq, "after" if same else "all"), nq))
             else:
-                nq = 1  # a contracted pair's primitives already make a long task
-                chunks = groups.chunks(lc, nq, "own" if metric and la == lc else "all")
-                lst, rows, first = groups.group_rows(lc, nq)
-                ids = groups.group_ids(la) if metric else None
-                arr[i] = _lib.PrimClass(la, lb, lc, n, p(pairs), p(chunks), p(lst), rows.ctypes.data, first.ctypes.data,
-                                        len(rows) - 1, groups.max_shells(lc), p(ids), 0 if ids is None else ids.numel(),
-                                        groups.prims[la][0] if metric else 0, int((la, lb, lc) in f32))
-        per = 0 if deriv or not new else int(L.dfb_prim_scratch(arr, len(new), PRIM_WAVE))
+                # one primitive per task: a contracted pair's primitives already make a long one
+                chunks, _n = groups.chunk_range(lc, 1, "own" if same else "all")
+                lst, rows, first_chunk, ng = groups.group_rows(lc, 1)
+                ids, nids = groups.group_ids(la) if metric else (0, 0)
+                recs.append((la, lb, lc, n, pairs, chunks, lst, rows, first_chunk, ng, groups.max_shells[lc], ids, nids,
+                             groups.prims[la][0] if metric else 0, int((la, lb, lc) in f32)))
+        cls, dtype = (_lib.GradClass, _GRAD_CLASS) if deriv else (_lib.PrimClass, _PRIM_CLASS)
+        arr = (cls * max(len(new), 1))()
+        if recs:
+            np.frombuffer(arr, dtype=dtype)[:] = recs
+        per = 0 if deriv or not new else int(_lib.lib().dfb_prim_scratch(arr, len(new), PRIM_WAVE))
         return arr, len(new), old, per
 
     def _int3c_work(self, X, strides, precision, groups=None, axs=None, byl=None):
