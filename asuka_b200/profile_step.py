@@ -77,7 +77,8 @@ def phases(eng: DFEngine, Cw: torch.Tensor, R: torch.Tensor, precision: str, X: 
 
 
 def class_times(eng, mol, top: int = 20, precision: str = "fp64") -> dict:
-    """Per-class device time of the 3c integrals and the 3c derivative contraction."""
+    """Per-class device time of the 3c integrals and the 3c derivative contraction on the shell-by-shell kernels
+    (what ``tune_classes`` tunes)."""
     import ctypes
     import os
     import sys
@@ -126,6 +127,48 @@ def class_times(eng, mol, top: int = 20, precision: str = "fp64") -> dict:
     return out
 
 
+def step_class_times(eng, top: int = 20, precision: str = "fp64") -> dict:
+    """Per-class device time of the 3c integrals and the 3c derivative contraction, on the kernels that a step of
+    this precision runs ("group" or "shell")."""
+    nao = eng.nao
+    s = (nao * nao, nao, 1)
+    X = torch.zeros((eng.naux, nao, nao), dtype=torch.float64, device="cuda")
+    g = torch.zeros((eng.natm, 3), dtype=torch.float64, device="cuda")
+    every = eng.classes3c
+    e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    out = {}
+    try:
+        for key in ("int3c", "deriv3c"):
+            res = []
+            for entry in every:
+                eng.classes3c = [entry]
+
+                def run():
+                    if key == "int3c":
+                        eng._run_int([eng._int3c_work(X, s, precision)])
+                    else:
+                        eng._run_deriv([eng._deriv3c_work(X, s, g, precision)], g)
+
+                run()
+                torch.cuda._sleep(1000000)  # the launches queue up behind it
+                e0.record()
+                for _ in range(3):
+                    run()
+                e1.record()
+                torch.cuda.synchronize()
+                la, lb, lc, pairs, auxs = entry
+                group = eng._plan("int" if key == "int3c" else "der", eng.groups, precision)[1]
+                res.append((e0.elapsed_time(e1) / 3, f"({la},{lb},{lc})", pairs.numel() * auxs.numel(),
+                            "group" if group else "shell"))
+            res.sort(reverse=True)
+            out[key] = {"total_ms": round(sum(r[0] for r in res), 3),
+                        "shell_ms": round(sum(r[0] for r in res if r[3] == "shell"), 3),
+                        "top": [[round(r[0], 3), r[1], r[2], r[3]] for r in res[:top]]}
+    finally:
+        eng.classes3c = every
+    return out
+
+
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--workload", default="w8", choices=sorted(WORKLOADS))
@@ -156,7 +199,7 @@ def main():
                               **{k: (round(v, 3) if isinstance(v, float) else v) for k, v in st.items()}}))
         return
     if args.classes:
-        print(json.dumps(class_times(eng, mol, precision=args.precision)))
+        print(json.dumps(step_class_times(eng, precision=args.precision)))
         return
     X = torch.empty((eng.naux, eng.nao, eng.nao), dtype=torch.float64, device="cuda")
     if args.only in ("int3c", "deriv3c", "metric", "deriv2c"):

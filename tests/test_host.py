@@ -88,8 +88,8 @@ def test_block_substitution_matches_triangular_solve():
     Y = torch.randn(n, 37, generator=g, dtype=torch.float64)
     ref = torch.linalg.solve_triangular(L, Y, upper=False)
     inv = linalg.diag_block_inverses(L)
-    # the inverses assembled from 64-row sub-blocks, and the per-block form (a block size that is
-    # not 64 * 2^k), against dense inverses
+    # inverses of whole 256-row blocks and of another block size (on the CPU both by a triangular
+    # solve per block), against dense inverses
     for nb, blocks in ((linalg.NB, inv), (100, linalg.diag_block_inverses(L, 100))):
         for i, r0 in enumerate(range(0, n, nb)):
             r1 = min(n, r0 + nb)
