@@ -147,6 +147,13 @@ def check(rc: int, what: str) -> None:
         raise RuntimeError(f"{what} failed ({rc}): {msg}")
 
 
+def current_stream(index: int | None = None) -> int:
+    """Handle of torch's current stream on a GPU (the current one by default)."""
+    import torch
+
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
+
+
 def ptr(t) -> int:
     """Device (or host) address of a torch tensor; 0 for None."""
     return 0 if t is None else int(t.data_ptr())

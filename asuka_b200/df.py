@@ -55,6 +55,7 @@ GRAD_THREADS, GRAD_BIG = 1 << 17, 1 << 20
 SEG_PRIMS = 8  # primitive pairs of a derivative task: contracted pairs are cut, so that no task outlasts the rest
 NROOTS_SLOTS = 11  # DFB_NROOTS_MAX + 1
 _SIDE_STREAMS: dict[int, list] = {}
+_SIDE_HANDLES: dict = {}  # device index -> ctypes array of the side streams' handles
 
 
 class ScratchHolder:
@@ -147,7 +148,7 @@ def _class_prec(code: int, kind: str, la: int, lb: int, lc: int) -> int:
 
 
 def _stream() -> int:
-    return int(torch.cuda.current_stream().cuda_stream)
+    return _lib.current_stream()
 
 
 def _as_soa(b) -> BasisCartSoA:
@@ -297,20 +298,22 @@ class DFEngine:
         return _SIDE_STREAMS[idx]
 
     def _fork(self):
-        """(main stream, side streams, ctypes array of their handles), the side streams ordered after the
-        current stream."""
-        main = torch.cuda.current_stream(self.device)
+        """(handle of the current stream, number of side streams, ctypes array of their handles), the side streams
+        ordered after the current stream."""
+        main = _lib.current_stream(self.device.index)
         if NSTREAMS <= 1:
-            return main, [main], (ctypes.c_void_p * 1)(int(main.cuda_stream))
-        side = self._streams()
-        arr = (ctypes.c_void_p * len(side))(*[int(st.cuda_stream) for st in side])
-        _lib.check(_lib.lib().dfb_fork(int(main.cuda_stream), arr, len(side)), "dfb_fork")
-        return main, side, arr
+            return main, 1, (ctypes.c_void_p * 1)(main)
+        idx = self.device.index if self.device.index is not None else torch.cuda.current_device()
+        arr = _SIDE_HANDLES.get(idx)
+        if arr is None:
+            arr = _SIDE_HANDLES[idx] = (ctypes.c_void_p * NSTREAMS)(*[int(st.cuda_stream) for st in self._streams()])
+        _lib.check(_lib.lib().dfb_fork(main, arr, NSTREAMS), "dfb_fork")
+        return main, NSTREAMS, arr
 
     def _join(self, fork) -> None:
-        main, side, arr = fork[:3]
-        if side[0] is not main:
-            _lib.check(_lib.lib().dfb_join(int(main.cuda_stream), arr, len(side)), "dfb_join")
+        main, n, arr = fork[:3]
+        if NSTREAMS > 1:
+            _lib.check(_lib.lib().dfb_join(main, arr, n), "dfb_join")
 
     @property
     def _i32(self):
@@ -611,13 +614,13 @@ class DFEngine:
         now = () if kind.endswith("2") else self.classes3c
         known = groups.plans.get(key)
         if known is not None:
-            entries, plan = known
-            if len(entries) == len(now) and all(a is b for a, b in zip(entries, now)):
+            ids, plan, _entries = known
+            if ids == [*map(id, now)]:  # of entries that the plan keeps alive
                 return plan
         if len(groups.plans) > 16:
             groups.plans.clear()
         plan = self._make_plan(kind, groups, shells, f32 or (), block)
-        groups.plans[key] = (tuple(now), plan)
+        groups.plans[key] = ([*map(id, now)], plan, tuple(now))
         return plan
 
     def _make_plan(self, kind: str, groups: AuxGroups, shells: bool, f32, block: bool):
@@ -732,16 +735,16 @@ class DFEngine:
         per = (max(w[4] for w in every) + 31) // 32 * 32
         rows = torch.empty(n * per, dtype=torch.float64, device=self.device)
         fork = (*self._fork(), rows)
-        _main, side, streams, _rows = fork
+        streams = fork[2]
         try:
             for batch in (works, then or []):
                 for bra, groups, arr, ncls, _per, out, (sP, sM, sN), rest in batch:
                     if ncls:
                         rc = L.dfb_prim_integrals(ctypes.byref(bra), ctypes.byref(groups.c), arr, ncls, _lib.ptr(out), sP,
-                                                  sM, sN, _lib.ptr(rows), rows.numel(), streams, len(side))
+                                                  sM, sN, _lib.ptr(rows), rows.numel(), streams, n)
                         _lib.check(rc, "dfb_prim_integrals")
                     for i, job in enumerate(rest):
-                        self._launch_int(*job)(int(side[i % n].cuda_stream))
+                        self._launch_int(*job)(streams[i % n])
                 if batch is works:
                     self._join(fork)
         except BaseException:
@@ -756,14 +759,14 @@ class DFEngine:
         if any(w[6] for w in works):
             self._slices_der = self._scratch_slices(True)
         fork = self._fork()
-        _main, side, streams = fork
+        streams = fork[2]
         for bra, groups, arr, ncls, bar, (sP, sM, sN), rest in works:
             if ncls:
                 rc = L.dfb_grad_contract(ctypes.byref(bra), ctypes.byref(groups.c), arr, ncls, _lib.ptr(bar), sP, sM, sN,
-                                         _lib.ptr(grad), self.natm, streams, len(side))
+                                         _lib.ptr(grad), self.natm, streams, n)
                 _lib.check(rc, "dfb_grad_contract")
             for i, job in enumerate(rest):
-                self._launch_deriv(*job)(int(side[i % n].cuda_stream))
+                self._launch_deriv(*job)(streams[i % n])
         self._join(fork)
 
     # ------------------------------------------------------------ overlapped phases of one step

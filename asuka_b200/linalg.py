@@ -92,7 +92,7 @@ def solve_lower_right_T(L: torch.Tensor, X: torch.Tensor, inv: list[torch.Tensor
 def _launch(device: torch.device, fn, *args) -> int:
     """fn(*args, the device's current stream) with that device current: a kernel is launched on the current
     device, and its stream has to belong to it."""
-    stream = int(torch.cuda.current_stream(device).cuda_stream)
+    stream = _lib.current_stream(device.index)
     if device.index in (None, torch.cuda.current_device()):
         return fn(*args, stream)
     with torch.cuda.device(device):

@@ -175,7 +175,6 @@ def test_launches_enter_the_tensors_device(monkeypatch):
     """The launch helper with recorded torch.cuda calls: the tensors' device is made current around the call
     when it is not, and the stream is that device's."""
     from contextlib import contextmanager
-    from types import SimpleNamespace as NS
 
     from asuka_b200 import linalg
 
@@ -189,7 +188,7 @@ def test_launches_enter_the_tensors_device(monkeypatch):
 
     monkeypatch.setattr(torch.cuda, "current_device", lambda: state["current"])
     monkeypatch.setattr(torch.cuda, "device", device)
-    monkeypatch.setattr(torch.cuda, "current_stream", lambda d: NS(cuda_stream=100 + d.index))
+    monkeypatch.setattr(linalg._lib, "current_stream", lambda index: 100 + index)
     for idx in (0, 1):
         assert linalg._launch(torch.device("cuda", idx), lambda x, st: (x, st, state["current"]), 7) == (7, 100 + idx, idx)
         assert state["current"] == 0

@@ -33,8 +33,7 @@ def test_calls_in_flight_have_their_own_rows(monkeypatch):
     eng = df.DFEngine.__new__(df.DFEngine)
     eng.device = torch.device("cpu")
     eng._scratch = df.ScratchHolder()
-    st = NS(cuda_stream=0)
-    monkeypatch.setattr(df.DFEngine, "_fork", lambda self: (st, [st] * 8, (ctypes.c_void_p * 8)()))
+    monkeypatch.setattr(df.DFEngine, "_fork", lambda self: (0, 8, (ctypes.c_void_p * 8)()))
     monkeypatch.setattr(df.DFEngine, "_join", lambda self, fork: None)
     out = torch.zeros(1)
     groups = NS(c=_lib.Groups())
