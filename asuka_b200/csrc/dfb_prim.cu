@@ -148,17 +148,22 @@ static long group_rows(const dfb_prim_class_t& c) {
     return most;
 }
 
-// A wave holds whole groups over a range of pair tiles: `target` doubles bound it unless one group over one
-// tile takes more.  The metric contracts pairs of groups: its waves hold all pairs, whose count grows with the
-// primitives of one l only.
+// A wave holds whole groups.  `target` doubles bound it unless one group takes more: then one group over all pairs up
+// to PRIM_OVER times the target, and over a range of pair tiles beyond (at least one tile).  Cutting the pairs costs
+// launches and short waves: integrals of 12 waters TZVP in blocks, where one group over all pairs is 1.0 to 1.7 of
+// 8 MB, 17.0 ms cut and 15.5 uncut.  The metric contracts pairs of groups: its waves hold all pairs, whose
+// count grows with the primitives of one l only.
+constexpr long PRIM_OVER = 4;
 extern "C" long dfb_prim_scratch(const dfb_prim_class_t* cls, int ncls, long target) {
     long need = 1;
     for (int i = 0; i < ncls; ++i) {
         const dfb_prim_class_t& c = cls[i];
         if (c.ngroup <= 0 || c.npair <= 0) continue;
-        const long tiles = ((long)c.npair + 31) / 32, one = tile_row(c) * (c.bra_groups ? tiles : 1);
-        const long least = group_rows(c) * one, all = c.rows[c.ngroup] * tile_row(c) * tiles;
-        long n = least > target ? least : target;
+        const long tiles = ((long)c.npair + 31) / 32, one = group_rows(c) * tile_row(c);
+        long n = one * tiles;
+        if (!c.bra_groups && n > PRIM_OVER * target) n = one > PRIM_OVER * target ? one : PRIM_OVER * target;
+        if (n < target) n = target;
+        const long all = c.rows[c.ngroup] * tile_row(c) * tiles;
         if (n > all) n = all;
         if (n > need) need = n;
     }
@@ -220,6 +225,7 @@ extern "C" int dfb_prim_integrals(const dfb_bra_t* bra, const dfb_groups_t* gr, 
             const long fit = big > 0 ? slice / (big * tile_row(c)) : tiles, grid = 65535L * (GRAD_THREADS / 32);
             step = tiles < fit ? tiles : fit;
             step = step < grid ? step : grid;
+            if (step > 0) step = (tiles + (tiles + step - 1) / step - 1) / ((tiles + step - 1) / step);  // equal ranges
         }
         if (step < 1)
             return set_error(DFB_ERR_INVALID, "class (%d,%d,%d) needs %ld scratch doubles per stream, %ld given", c.la, c.lb,

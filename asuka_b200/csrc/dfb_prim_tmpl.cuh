@@ -4,7 +4,7 @@
 // once per (AO pair, primitive) into the rows of W (tiles of 32 pairs, 256-byte segments), and
 // k_prim_out contracts a group's rows to its shells, applies the horizontal recurrence and writes
 // the 3c tensor (k_prim_out2: both sides of the metric).  A wave takes whole groups over a range of pair tiles,
-// so that its rows stay within the scratch given per stream (8 MB, or one group over one tile).
+// so that its rows stay within the scratch given per stream (8 to 32 MB, or one group over one tile).
 //
 // (H2O)8/ma-TZVP, 416 AO / 1824 aux: 3c integrals 5.5 ms with one evaluation per shell, 4.75 ms here, of which
 // the contraction k_prim_out takes most (its blocks wait on dependent loads); metric 0.80 -> 0.33 ms.

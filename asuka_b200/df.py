@@ -39,7 +39,7 @@ _DATA = os.path.join(os.path.dirname(os.path.abspath(__file__)), "data")
 _TABLE_READY: set[int] = set()
 PRIM_SCREEN = 1e-20  # primitive-pair magnitude bound below which a pair is skipped (0 = evaluate all)
 NSTREAMS = int(os.environ.get("DFB_STREAMS", "8"))  # side streams for per-class launches (2/4/6/8 measured: 8 fastest)
-# Doubles of primitive integrals per stream and wave of a class (8 MB; one group over 32 pairs where that is more):
+# Doubles of primitive integrals per stream and wave of a class (8 MB; one group up to 32 MB, or over 32 pairs):
 # eight streams then stay within L2.  3c integrals at 8 / 64 MB: (H2O)8 4.86 / 4.96 ms, decane 1.88 / 1.86,
 # (H2O)3 QZVP 7.85 / 7.77; scratch 71 / 535 MB
 PRIM_WAVE = 1 << 20

@@ -269,7 +269,7 @@ typedef struct {
 } dfb_prim_class_t;
 
 /*
- * Doubles of scratch per stream for waves of about `target` doubles: at most target, or one group over 32 AO pairs
+ * Doubles of scratch per stream for waves of about `target` doubles: at most 4 target, or one group over 32 AO pairs
  * (metric: over all primitives of the bra l) where that is more.
  */
 long dfb_prim_scratch(const dfb_prim_class_t *cls, int ncls, long target);

@@ -100,8 +100,8 @@ def test_captured_call_outlives_larger_ones():
 @pytest.mark.parametrize("l", [(0, 0, 0), (1, 1, 2), (2, 1, 4), (4, 4, 6)])
 @pytest.mark.parametrize("npair", [1, 32, 33, 5000])
 def test_rows_stay_within_the_target(l, npair):
-    """Scratch of one class on the host: the target, unless all rows take less or one group over one tile of 32
-    pairs takes more; the pair count does not enter otherwise."""
+    """Scratch of one class on the host: the target, or one group over all pairs up to four times as much, or one
+    group over one tile of 32 pairs, unless all rows take less; the pair count does not enter otherwise."""
     import numpy as np
 
     from asuka_b200 import _lib
@@ -116,8 +116,10 @@ def test_rows_stay_within_the_target(l, npair):
     c = _lib.PrimClass(la, lb, lc, npair, 0, 0, 0, rows.ctypes.data, rows.ctypes.data, 3, 2, 0, 0, 0, 0)
     for target in (1, 1 << 16, 1 << 20, 1 << 30):
         need = L.dfb_prim_scratch(ctypes.byref(c), 1, target)
-        assert need <= max(target, 22 * tile)
-        assert need == min(max(target, 22 * tile), 30 * tile * -(-npair // 32))
+        tiles = -(-npair // 32)
+        assert need <= max(4 * target, 22 * tile)
+        group = 22 * tile * tiles if 22 * tile * tiles <= 4 * target else max(4 * target, 22 * tile)
+        assert need == min(max(target, group), 30 * tile * tiles)
     c.bra_groups = 1  # metric: all pairs
     need = L.dfb_prim_scratch(ctypes.byref(c), 1, 1)
     assert need == 22 * tile * -(-npair // 32)
