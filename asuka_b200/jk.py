@@ -22,6 +22,7 @@ from __future__ import annotations
 
 import torch
 
+from . import _lib
 from . import linalg as _la
 from . import tc as _tc
 
@@ -48,7 +49,7 @@ def _half_rows(BQ: torch.Tensor, nocc: int, q_block: int) -> int:
     if q_block == 0:
         raise ValueError("q_block must be > 0")
     naux, nao, _ = BQ.shape
-    if not BQ.is_contiguous():  # a block of such factors is copied, too
+    if naux <= q_block or not BQ.is_contiguous():  # a block of such factors is copied, too
         return q_block
     return max(q_block, min(naux, min(HALF_ELEMS, BQ.numel() // 4) // max(nao * nocc, 1)))
 
@@ -180,8 +181,12 @@ class DFJKWorkspace:
         return int(q_block)
 
     def _run(self, st: torch.cuda.Stream, sync: bool, fn):
-        with torch.cuda.stream(st):
+        here = torch.cuda.current_device()
+        if st.device_index == here and st.cuda_stream == _lib.current_stream(here):
             fn()
+        else:
+            with torch.cuda.stream(st):
+                fn()
         if sync:
             st.synchronize()
 

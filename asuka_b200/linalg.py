@@ -119,10 +119,10 @@ def _observed(*tensors: torch.Tensor) -> bool:
 def _kernel_update(W: torch.Tensor, out: torch.Tensor) -> bool:
     """True when the exchange kernel can take W (naux, nao, nocc) and out: FP64 on one GPU, out a row-major
     (nao, nao) matrix.  Its pointers carry neither a type nor a device, so everything else stays with torch."""
-    return (W.is_cuda and out.device == W.device and W.dtype == torch.float64 and out.dtype == torch.float64
-            and tuple(out.shape) == (W.shape[1], W.shape[1]) and (out.stride(1) == 1 and out.stride(0) >= W.shape[1]
-                                                                  or out.shape[0] <= 1)
-            and not (W.is_neg() or out.is_neg()))
+    n, f64 = W.shape[1], torch.float64
+    if not (W.is_cuda and W.dtype is f64 and out.dtype is f64 and out.device == W.device and out.shape == (n, n)):
+        return False
+    return (out.stride(1) == 1 and out.stride(0) >= n or n <= 1) and not (W.is_neg() or out.is_neg())
 
 
 @functools.lru_cache(maxsize=256)
