@@ -271,12 +271,14 @@ class DFEngine:
         self._pair_static = _PairStatic(ao, self.sp)
         self._build_ao_pairs(ao.shell_cxyz)
         self._build_pair_tables()
+        if os.environ.get("DFB_DISABLE_TMPL"):
+            self.classes2c  # noqa: B018  (lists of the shell metric kernels, before any capture)
 
     # ------------------------------------------------------------ class lists
     @property
     def classes2c(self):
         """Metric classes of the shell-by-shell kernels: (lP, lQ, P list, Q list) over the unordered aux shell
-        pairs oriented l(P) >= l(Q); built when first asked for."""
+        pairs oriented l(P) >= l(Q); built when first asked for (with DFB_DISABLE_TMPL set, by the constructor)."""
         if self._classes2c is None:
             aux_l = self.aux.shell_l
             Pi, Qi = np.tril_indices(self.aux.nshell)
@@ -438,10 +440,13 @@ class DFEngine:
             n = L.dfb_rys_scratch_doubles(la, lb, lc, pairs.numel() * auxs.numel(), int(deriv))
             _lib.check(0 if n >= 0 else int(n), "dfb_rys_scratch_doubles")
             need = max(need, n)
-        for lp, lq, P, Q in self.classes2c:
-            n = L.dfb_rys_scratch_doubles(lp, 0, lq, P.numel(), int(deriv))
-            _lib.check(0 if n >= 0 else int(n), "dfb_rys_scratch_doubles")
-            need = max(need, n)
+        ls, count = np.unique(self.aux.shell_l, return_counts=True)
+        for i, lp in enumerate(ls.tolist()):  # unordered aux shell pairs, counted without their lists
+            for lq, m in zip(ls[:i + 1].tolist(), count[:i + 1].tolist()):
+                pairs = int(count[i]) * m if lq < lp else m * (m + 1) // 2
+                n = L.dfb_rys_scratch_doubles(lp, 0, lq, pairs, int(deriv))
+                _lib.check(0 if n >= 0 else int(n), "dfb_rys_scratch_doubles")
+                need = max(need, n)
         cache[key] = need
         return self._scratch.get(need * copies, self.device)
 

@@ -168,3 +168,61 @@ def test_rule_of_the_zeros(monkeypatch, layout, share, blocks):
     X = torch.ones(8)
     eng._clear_dropped(X, (16, 4, 1) if layout == "Qmn" else (1, 32, 8), 8)
     assert bool(calls) == blocks and bool((X == 0).all()) != blocks
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", ["whole", "edited", "h shell", "generic"])
+def test_first_call_under_capture(monkeypatch, form):
+    """The first integral, metric and derivative calls of an engine, recorded into a graph, for the classes of the
+    group kernels and for those that stay on the shell kernels: nothing is uploaded by a call."""
+    import dataclasses
+
+    import numpy as np
+
+    from asuka_b200 import basis as bm
+    from asuka_b200 import df, geometry as geo
+
+    if form == "generic":
+        monkeypatch.setenv("DFB_DISABLE_TMPL", "1")
+    mol = geo.n2()
+    atoms = list(mol.atoms_bohr)
+    ao, aux = bm.pack_basis(atoms, mol.basis, "ao"), bm.pack_basis(atoms, mol.basis, "aux")
+    if form == "h shell":
+        ao = dataclasses.replace(
+            ao, shell_cxyz=np.vstack([ao.shell_cxyz, ao.shell_cxyz[:1]]),
+            shell_prim_start=np.append(ao.shell_prim_start, ao.prim_exp.size).astype(np.int32),
+            shell_nprim=np.append(ao.shell_nprim, 1).astype(np.int32), shell_l=np.append(ao.shell_l, 5).astype(np.int32),
+            shell_ao_start=np.append(ao.shell_ao_start, ao.nao).astype(np.int32), prim_exp=np.append(ao.prim_exp, 0.9),
+            prim_coef=np.append(ao.prim_coef, 0.3), shell_atom=np.append(ao.shell_atom, 0).astype(np.int32))
+
+    def engine():
+        eng = df.DFEngine(ao, aux)
+        if form == "edited":
+            eng.classes3c = [(a, b, c, p.clone(), x) for a, b, c, p, x in eng.classes3c]
+        return eng
+
+    ref = engine()
+    bar = torch.ones((ref.naux, ref.nao, ref.nao), dtype=torch.float64, device="cuda")
+    bar2 = torch.ones((ref.naux, ref.naux), dtype=torch.float64, device="cuda")
+
+    def calls(eng, X, V, g):
+        eng.int3c("Qmn", out=X)
+        eng.metric(out=V)
+        eng.deriv3c(bar, g)
+        eng.deriv2c(bar2, g)
+
+    def outputs(eng):
+        return (torch.zeros_like(bar), torch.zeros_like(bar2), torch.zeros((eng.natm, 3), dtype=torch.float64, device="cuda"))
+
+    want = outputs(ref)
+    calls(ref, *want)
+    eng = engine()
+    got = outputs(eng)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        calls(eng, *got)
+    graph.replay()
+    torch.cuda.synchronize()
+    for a, b in zip(got, want):
+        assert float((a - b).abs().max()) <= 1e-12 * float(b.abs().max())
